@@ -154,7 +154,7 @@ struct caffe_dev {
     double* paN = nullptr;
     double* paT = nullptr;
     double* pb = nullptr;
-    KspWork kw;
+    KspWork kw = {};
     IbState ibs;
     // learned preconditioner of the p' solve
     LearnedWork lw;
@@ -256,7 +256,7 @@ struct caffe_dev {
         gh.cell = ibs.gCell;
         gh.col = ibs.gCol;
         gh.val = which == 0 ? ibs.gValMom : ibs.gValP;
-        gh.bits = ibs.bits;
+        gh.words = ibs.words;
         return gh;
     }
     Op7 momOp() const {
@@ -364,9 +364,7 @@ int fill(caffe_dev* h, double* dst, int planes, double a, double b = 0., double 
 // constant vector is its null space) and its right-hand side carries a round-off
 // component along it that no Krylov method can remove; the solver then projects the
 // right-hand side onto the range first (the CPU oracle does the same).
-// deepest relative residual reduction an FP32 inner solve of the mixed-precision form aims for
-// (later inner solves only aim for the factor still missing)
-constexpr double MIXED_INNER_RTOL = 1e-6;
+// deepest relative residual reduction an FP32 inner solve of the learned form aims for
 constexpr double LEARNED_INNER_RTOL = 1e-5;
 
 int p_singular(const caffe_dev* h) {
@@ -417,11 +415,11 @@ int ph_solve_pcorr(caffe_dev* h) {
                            project, h->netMode, h->kw.out, h->st, h->cs.p_atol);
         if (!rc) rc = ksp_fallback_sym(A, method, h->pb, h->pc, h->L, h->kw, h->cs.p_rtol, h->cs.maxit, h->st, 0,
                                        &h->kw.out->status[0], &h->acc->fallbacks, h->cs.p_atol);
-    } else if (h->cs.p_form == CAFFE_P_MIXED) {
-        // FP32 inner solves inside FP64 refinement; the plain FP64 solve re-runs on the device
-        // when the refinement does not reach the tolerance
-        rc = ksp_mixed_sym(A, method, h->pb, h->pc, h->L, h->kw, h->cs.p_rtol, h->cs.maxit, MIXED_INNER_RTOL, h->st, project,
-                           h->cs.p_atol);
+    } else if (h->cs.p_form == CAFFE_P_MIXED && sym) {
+        // FP32 CG inside FP64 refinement (whichever method the case names: the system is symmetric);
+        // the plain FP64 solve re-runs on the device when the refinement does not reach the
+        // tolerance.  Systems with ghost rows take the FP64 BiCGStab below (krylov.cu)
+        rc = ksp_mixed_sym(A, h->pb, h->pc, h->L, h->kw, h->cs.p_rtol, h->cs.maxit, h->st, project, h->cs.p_atol);
         if (!rc) rc = ksp_fallback_sym(A, method, h->pb, h->pc, h->L, h->kw, h->cs.p_rtol, h->cs.maxit, h->st, 0,
                                        &h->kw.out->status[0], &h->acc->fallbacks, h->cs.p_atol);
     } else if (method == CAFFE_KSP_CG_JACOBI) {
@@ -674,18 +672,16 @@ int caffe_dev_create(const double* nodes, int nNI, int nNJ, int nNK, const caffe
     h->kw.p[0] = h->cell(3); h->kw.p[1] = h->cell(3);
     h->kw.v[0] = h->cell(3); h->kw.v[1] = h->cell(3);
     h->kw.t = h->cell(3); h->kw.invD = h->cell(1);
-    if (cs->p_form == CAFFE_P_MIXED || cs->p_form == CAFFE_P_LEARNED_MIXED) {
-        for (int q = 0; q < 2; ++q) { h->kw.fr[q] = h->fcell(); h->kw.fw[q] = h->fcell(); h->kw.fs[q] = h->fcell(); h->kw.fv[q] = h->fcell(); }
-        h->kw.fp = h->fcell(); h->kw.fe = h->fcell(); h->kw.ft = h->fcell(); h->kw.finvD = h->fcell();
-        for (int q = 0; q < 4; ++q) h->kw.fA[q] = h->fcell();
-        bool ok = h->kw.fp && h->kw.fe && h->kw.ft && h->kw.finvD;
-        for (int q = 0; q < 2; ++q) ok = ok && h->kw.fr[q] && h->kw.fw[q] && h->kw.fs[q] && h->kw.fv[q];
-        for (int q = 0; q < 4; ++q) ok = ok && h->kw.fA[q];
+    // CG does not use the three planes of rp: they hold its scaled operator
+    for (int q = 0; q < 3; ++q) h->kw.cs[q] = h->kw.rp ? h->kw.rp + q * L.PS : nullptr;
+    if (cs->p_form == CAFFE_P_MIXED) {
+        h->kw.fr = h->fcell(); h->kw.fq = h->fcell(); h->kw.fp = h->fcell(); h->kw.fe = h->fcell(); h->kw.fd = h->fcell();
+        for (int q = 0; q < 3; ++q) h->kw.fB[q] = h->fcell();
+        bool ok = h->kw.fr && h->kw.fq && h->kw.fp && h->kw.fe && h->kw.fd;
+        for (int q = 0; q < 3; ++q) ok = ok && h->kw.fB[q];
         if (!ok) { set_error("device allocation failed (mixed-precision workspace)"); return fail(); }
     }
-    int nsm = 0;
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
-    h->kw.partials = h->dalloc<double>((size_t)2 * 8 * 8 * (nsm > 0 ? nsm : 256));
+    h->kw.partials = h->dalloc<double>(krylov_partial_doubles());
     h->kw.out = h->dalloc<KspOut>(1);
     h->chunkMax = h->dalloc<double>((size_t)(L.N / 1024 + 2));
     h->acc = h->dalloc<StepAcc>(1);
@@ -1189,9 +1185,10 @@ int caffe_ksp7_solve_device(int nI, int nJ, int nK, const double* d_coef7, const
     // the second plane of r as its double buffer)
     w.r = cellbuf(3); w.rp = cellbuf(3); w.p[0] = cellbuf(3); w.p[1] = cellbuf(3);
     w.v[0] = cellbuf(3); w.v[1] = cellbuf(3); w.t = cellbuf(3); w.invD = cellbuf(1);
+    for (int q = 0; q < 3; ++q) w.cs[q] = w.rp ? w.rp + q * L.PS : nullptr;
     void* part = nullptr;
     void* outp = nullptr;
-    bool ok = cudaMalloc(&part, 2 * 8 * 8 * 1024 * sizeof(double)) == cudaSuccess && cudaMalloc(&outp, sizeof(KspOut)) == cudaSuccess;
+    bool ok = cudaMalloc(&part, krylov_partial_doubles() * sizeof(double)) == cudaSuccess && cudaMalloc(&outp, sizeof(KspOut)) == cudaSuccess;
     if (part) tmp.push_back(part);
     if (outp) tmp.push_back(outp);
     for (int q = 0; q < 7; ++q) ok = ok && a7[q];
@@ -1207,7 +1204,7 @@ int caffe_ksp7_solve_device(int nI, int nJ, int nK, const double* d_coef7, const
     }
     if (cudaMemcpyAsync(b, d_b, L.N * sizeof(double), cudaMemcpyDeviceToDevice, st) != cudaSuccess) { cleanup(); set_error("rhs copy failed"); return 1; }
     A.nI = L.nI; A.nIJ = L.nIJ;
-    A.gh.n = 0; A.gh.cell = nullptr; A.gh.col = nullptr; A.gh.val = nullptr; A.gh.bits = nullptr;
+    A.gh.n = 0; A.gh.cell = nullptr; A.gh.col = nullptr; A.gh.val = nullptr; A.gh.words = nullptr;
     int rc;
     if (method == CAFFE_KSP_CG_JACOBI) rc = ksp_cg7(A, b, x, L, w, rtol, maxit, st);
     else rc = ksp_bicgstab(A, 1, b, x, L, w, rtol, maxit, st);

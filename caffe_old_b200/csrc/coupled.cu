@@ -64,7 +64,7 @@ struct caffe_coupled {
     double* b = nullptr;
     double* x = nullptr;
     double* contMax = nullptr;
-    KspWork kw;
+    KspWork kw = {};
     int iters = 0, status = 0;
     double relres = 0.;
 
@@ -556,7 +556,7 @@ int caffe_coupled_create(const double* nodes, int nNI, int nNJ, int nNK, const c
     h->kw.p[0] = h->dalloc<double>(n4); h->kw.p[1] = h->dalloc<double>(n4);
     h->kw.v[0] = h->dalloc<double>(n4); h->kw.v[1] = h->dalloc<double>(n4);
     h->kw.t = h->dalloc<double>(n4); h->kw.invD = h->dalloc<double>(n4);
-    h->kw.partials = h->dalloc<double>((size_t)2 * 8 * 8 * 1024);
+    h->kw.partials = h->dalloc<double>(krylov_partial_doubles());
     h->kw.out = h->dalloc<KspOut>(1);
     for (void* q : h->allocs)
         if (!q) { set_error("device allocation failed"); return fail(); }

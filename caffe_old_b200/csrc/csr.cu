@@ -96,7 +96,7 @@ extern "C" int caffe_csr_solve(int n, const int* row_ptr, const int* col, const 
     w.v[0] = d.get<double>(n); w.v[1] = d.get<double>(n);
     w.t = d.get<double>(n);
     w.invD = d.get<double>(n);
-    w.partials = d.get<double>((size_t)2 * 8 * 8 * 1024);
+    w.partials = d.get<double>(krylov_partial_doubles());
     w.out = d.get<KspOut>(1);
     bool ok = dptr && dcol && dval && ddiag && db && dx && w.r && w.rp && w.p[0] && w.p[1] && w.v[0] && w.v[1] && w.t && w.invD &&
               w.partials && w.out;

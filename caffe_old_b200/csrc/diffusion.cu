@@ -50,7 +50,7 @@ struct caffe_diffusion {
     double* b = nullptr;
     double* x = nullptr;
     double* resMax = nullptr;
-    KspWork kw;
+    KspWork kw = {};
     int iters = 0;
     double relres = 0.;
 
@@ -274,7 +274,7 @@ int launch_solve(caffe_diffusion* h) {
     Op7 A;
     for (int q = 0; q < 7; ++q) A.a[q] = h->a[q];
     A.nI = h->L.nI; A.nIJ = h->L.nIJ;
-    A.gh.n = 0; A.gh.cell = nullptr; A.gh.col = nullptr; A.gh.val = nullptr; A.gh.bits = nullptr;
+    A.gh.n = 0; A.gh.cell = nullptr; A.gh.col = nullptr; A.gh.val = nullptr; A.gh.words = nullptr;
     if (h->method == CAFFE_KSP_CG_JACOBI) return ksp_cg7(A, h->b, h->x, h->L, h->kw, h->rtol, h->maxit, h->st);
     return ksp_bicgstab(A, 1, h->b, h->x, h->L, h->kw, h->rtol, h->maxit, h->st);
 }
@@ -351,10 +351,11 @@ int caffe_diffusion_create(const double* nodes, int nNI, int nNJ, int nNK, const
     h->b = h->cell(1); h->x = h->cell(1);
     h->resMax = h->dalloc<double>(1);
     std::memset(&h->kw, 0, sizeof(h->kw));
-    h->kw.r = h->cell(2); h->kw.rp = h->cell(1);
+    h->kw.r = h->cell(2); h->kw.rp = h->cell(3);
     h->kw.p[0] = h->cell(1); h->kw.p[1] = h->cell(1); h->kw.v[0] = h->cell(1); h->kw.v[1] = h->cell(1);
     h->kw.t = h->cell(1); h->kw.invD = h->cell(1);
-    h->kw.partials = h->dalloc<double>((size_t)2 * 8 * 8 * 1024);
+    for (int q = 0; q < 3; ++q) h->kw.cs[q] = h->kw.rp ? h->kw.rp + q * h->L.PS : nullptr;
+    h->kw.partials = h->dalloc<double>(krylov_partial_doubles());
     h->kw.out = h->dalloc<KspOut>(1);
     for (void* p : h->allocs)
         if (!p) { set_error("device allocation failed"); return fail(); }

@@ -156,7 +156,7 @@ __global__ void ghost_flag_kernel(Lat L, const uint8_t* fld, uint8_t* status, in
     }
 }
 
-__global__ void ghost_list_kernel(Lat L, const uint8_t* status, const int* chunkOffset, int* gCell, uint32_t* bits) {
+__global__ void ghost_list_kernel(Lat L, const uint8_t* status, const int* chunkOffset, int* gCell, uint2* words) {
     long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     bool isG = c < L.N && status[c] == ST_GHOST;
     unsigned m = __ballot_sync(0xffffffffu, isG);
@@ -166,10 +166,10 @@ __global__ void ghost_list_kernel(Lat L, const uint8_t* status, const int* chunk
     __syncthreads();
     int base = chunkOffset[blockIdx.x];
     for (int q = 0; q < w; ++q) base += warpCount[q];
+    if (lane == 0 && c < L.N) words[c >> 5] = make_uint2(m, (unsigned)base);   // a warp's cells are one word's
     if (isG) {
         int idx = base + __popc(m & ((1u << lane) - 1u));
         gCell[idx] = (int)c;
-        atomicOr(bits + (c >> 5), 1u << (c & 31));
     }
 }
 
@@ -267,11 +267,11 @@ int ib_create(IbState& s, const Lat& L, uint8_t*& status, const Alloc& alloc, cu
     (void)st;
     status = reinterpret_cast<uint8_t*>(alloc((size_t)L.N));
     s.nChunks = (L.N + 1023) / 1024;
-    s.bits = reinterpret_cast<uint32_t*>(alloc(sizeof(uint32_t) * (size_t)(L.N / 32 + 2)));
+    s.words = reinterpret_cast<uint2*>(alloc(sizeof(uint2) * (size_t)(L.N / 32 + 2)));
     s.chunkCount = reinterpret_cast<int*>(alloc(sizeof(int) * (size_t)(s.nChunks + 1)));
     s.chunkOffset = reinterpret_cast<int*>(alloc(sizeof(int) * (size_t)(s.nChunks + 1)));
     s.err = reinterpret_cast<int*>(alloc(sizeof(int) * 4));
-    if (!status || !s.bits || !s.chunkCount || !s.chunkOffset || !s.err) { set_error("IB allocation failed"); return 1; }
+    if (!status || !s.words || !s.chunkCount || !s.chunkOffset || !s.err) { set_error("IB allocation failed"); return 1; }
     return 0;
 }
 
@@ -301,7 +301,7 @@ int ib_setup(IbState& s, const Geo& g, const caffe_case& cs, const double* d_xyz
     s.gValMom = reinterpret_cast<double*>(alloc(sizeof(double) * 9 * (size_t)cap));
     s.gValP = reinterpret_cast<double*>(alloc(sizeof(double) * 9 * (size_t)cap));
     if (!s.gCell || !s.gCol || !s.gValMom || !s.gValP) { set_error("IB allocation failed"); return 1; }
-    ghost_list_kernel<<<(unsigned)s.nChunks, 1024, 0, st>>>(L, status, s.chunkOffset, s.gCell, s.bits);
+    ghost_list_kernel<<<(unsigned)s.nChunks, 1024, 0, st>>>(L, status, s.chunkOffset, s.gCell, s.words);
     CB_CHECK_LAUNCH();
     if (s.nGhost > 0) {
         ghost_rows_kernel<<<grid_for(s.nGhost, 64), 64, 0, st>>>(g, d_xyz, status, s.nGhost, s.gCell, cs.ib_center[0], cs.ib_center[1],

@@ -14,7 +14,7 @@ struct IbState {
     int* gCol = nullptr;     // 9 per ghost: own cell, then the 8 stencil cells (-1 = dropped)
     double* gValMom = nullptr;
     double* gValP = nullptr;
-    uint32_t* bits = nullptr;
+    uint2* words = nullptr;  // per 32 cells: ghost bits, and how many ghost cells come before
     int* chunkCount = nullptr;
     int* chunkOffset = nullptr;
     int* err = nullptr;      // device error flag of the stencil kernel

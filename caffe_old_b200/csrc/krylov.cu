@@ -23,21 +23,392 @@
 // from others are not stored: CG's search direction p = z + beta p_old and BiCGStab's
 // p = r + beta (p_old - omega v) and s = r - alpha v are recomputed at the stencil
 // neighbours instead of costing an extra pass and barrier.
-#include <cooperative_groups.h>
+#include <algorithm>
 #include <cstring>
+#include "cg_scaled.cuh"
+#include "gridred.cuh"
 #include "krylov.cuh"
 #include "stencil.cuh"
 
 #define CAFFE_KSP_CG_JACOBI_INT 2   // caffe_ksp value of Jacobi-CG (include/caffe_b200.h)
 
-namespace cg = cooperative_groups;
-
 namespace cb {
 
+__device__ __forceinline__ double ldcg(const double* p) { return *p; }   // coherent load after a grid barrier
+
+template <class Op>
+__global__ void inv_diag_kernel(Op A, long long N, double* invD, double* slots) {
+    gr_clear(slots);
+    long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (c >= N) return;
+    double dg = diag_of(A, c);
+    invD[c] = dg != 0. ? 1. / dg : 1.;
+}
+
+template <class Op>
+__device__ __forceinline__ void sym_row(const Op& A, long long c, double& aE, double& aN, double& aT, bool& ok);
+template <>
+__device__ __forceinline__ void sym_row(const OpSym& A, long long c, double& aE, double& aN, double& aT, bool& ok) {
+    aE = A.aE[c]; aN = A.aN[c]; aT = A.aT[c];
+}
+template <>
+__device__ __forceinline__ void sym_row(const Op7& A, long long c, double& aE, double& aN, double& aT, bool& ok) {
+    aE = A.a[1][c]; aN = A.a[3][c]; aT = A.a[5][c];
+}
+// the west / south / bottom entries of row c equal the east / north / top ones of its neighbours
+// (an entry whose neighbour lies outside the lattice is zero)
+__device__ __forceinline__ bool row_symmetric(const OpSym&, long long, long long) { return true; }
+__device__ __forceinline__ bool row_symmetric(const Op7& A, long long c, long long) {
+    const double w = c >= 1 ? A.a[1][c - 1] : 0., s = c >= A.nI ? A.a[3][c - A.nI] : 0., b = c >= A.nIJ ? A.a[5][c - A.nIJ] : 0.;
+    return A.a[2][c] == w && A.a[4][c] == s && A.a[6][c] == b;
+}
+
+// Planes of B = sigma S A S (cg_scaled.cuh): S and the east, north and top off-diagonals.  general
+// (zero on entry) is set when the scaled form does not apply.
+template <class Op, class T>
+__global__ void scale_kernel(Op A, long long N, double* S, T* E, T* Nn, T* U, int* general, double* slots) {
+    gr_clear(slots);
+    long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (c >= N) return;
+    const double d0 = diag_of(A, 0), d = diag_of(A, c);
+    bool ok = (d0 > 0. && d > 0.) || (d0 < 0. && d < 0.);
+    double aE, aN, aT;
+    sym_row(A, c, aE, aN, aT, ok);
+    ok = ok && row_symmetric(A, c, N);
+    const double sg = d0 > 0. ? 1. : -1., s = 1. / sqrt(fabs(d));
+    auto off = [&](double a, long long e) {   // a = 0 beyond the lattice's end
+        return a == 0. ? 0. : e < N ? sg * a * s / sqrt(fabs(diag_of(A, e))) : __longlong_as_double(0x7ff8000000000000ll);
+    };
+    const double bE = off(aE, c + 1), bN = off(aN, c + A.nI), bT = off(aT, c + A.nIJ);
+    ok = ok && s == s && bE == bE && bN == bN && bT == bT;
+    S[c] = s; E[c] = (T)bE; Nn[c] = (T)bN; U[c] = (T)bT;
+    if (!ok) *general = 1;
+}
+
+struct KArgs {
+    const double* b;
+    double* x;
+    double* r;
+    double* s;     // BiCGStab
+    double* rp;
+    double* p[2];
+    double* v[2];
+    double* t;
+    const double* invD;
+    double* partials;
+    KspOut* out;
+    long long N, PS;
+    double rtol;
+    double atol;   // absolute floor: converged when ||b - A x|| <= max(rtol ||b||, atol)
+    int maxit;
+    int project;   // remove the mean of b first (singular all-Neumann pressure systems)
+    // fallback mode: when skip_if_ok is set the launch returns at once unless the status
+    // it points to (the previous solve's) is non-zero; fallbacks counts the launches that ran
+    const int* skip_if_ok;
+    int* fallbacks;
+    // CG: the scaled form's planes (1 / sqrt|d| in invD); null where only the general form runs
+    double* cs[3];
+};
+
+// Whether the scaled CG may run, decided on the device by scale_kernel: every diagonal entry of
+// one sign and, for seven separate coefficient planes, a symmetric matrix.
+__device__ __forceinline__ bool scaled_form(const KspOut* o) { return o->general == 0; }
+
+// Remove the mean of b (one plane), in place; every block computes the same mean.  Twice: where b was
+// almost a constant, what the first pass leaves is as much the rounding of that mean as b, and a
+// component along the null space that no iteration can remove makes CG diverge once r is down to it.
+__device__ __forceinline__ void project_mean(GridRed& grid, double* b, long long N, long long t0, long long T) {
+    for (int pass = 0; pass < 2; ++pass) {
+        double s[1] = {0.};
+        for (long long c = t0; c < N; c += T) s[0] += b[c];
+        double tot[1];
+        grid.sum<1>(s, tot);
+        double mean = tot[0] / (double)N;
+        for (long long c = t0; c < N; c += T) b[c] = b[c] - mean;
+    }
+    // the projected b is read at stencil neighbours owned by other blocks right after this
+    // (CG forms w = A D^-1 b): every block's subtraction must be visible first
+    grid.sync();
+}
+
+// ------------------------------------------------------------------ BiCGStab
+// Right-preconditioned BiCGStab (van der Vorst 1992) with two sweeps and two grid reductions per
+// iteration.  The vectors are stored as D^-1 times themselves (R, S, T, P, V for r, s, t, p, v), the form in
+// which the operator takes them, so that no 1/d is read at the stencil neighbours:
+//   sweep 1:  x += alpha P + omega S;  R = S - omega T;  P' = R + beta (P - omega V);  v = A P';  (rp, v)
+//   sweep 2:  S = R - alpha V;  t = A S;  (t, s), (t, t), (rp, s), (rp, t), (s, s)
+// The last sums give omega and, as r = s - omega t, the next rho = (rp, s) - omega (rp, t) and
+// (r, r) = (s, s) - 2 omega (t, s) + omega^2 (t, t) without a third sweep and reduction.  P' and S
+// are formed at the stencil neighbours from the stored vectors; P and V are double-buffered.
+// At a check (the recursive norm meets the tolerance, maxit, a breakdown) x takes the half-finished
+// iteration's update and the true residual decides, as in CG.
+// y = A f for W cells from c on; f.vec(e, o): values of W cells from e on, f.one(q, e): of one cell
+template <int NR, int W, class Op, class F>
+__device__ __forceinline__ void apply_w(const Op& A, long long c, F&& f, double (&y)[NR][W]) {
+    static_assert(W == 1, "only the symmetric operator has a group form");
+    double t[NR];
+    apply<NR>(A, c, [&](int q, long long e) { return f.one(q, e); }, t);
+#pragma unroll
+    for (int q = 0; q < NR; ++q) y[q][0] = t[q];
+}
+template <int NR, int W, class F>
+__device__ __forceinline__ void apply_w(const OpSym& A, long long c, F&& f, double (&y)[NR][W]) {
+    double o[W], n[W], s[W], t[W], b[W], kP[W], kE[W], kN[W], kS[W], kT[W], kB[W];
+    const uint2 gw = A.gh.n > 0 ? __ldg(A.gh.words + (c >> 5)) : make_uint2(0u, 0u);
+    f.vec(c, o);
+    f.vec(c + A.nI, n); f.vec(c - A.nI, s);
+    f.vec(c + A.nIJ, t); f.vec(c - A.nIJ, b);
+    const double w = f.one(0, c - 1), e = f.one(0, c + W), kw = A.aE[c - 1];
+    ldw<double, W>(A.aP + c, kP); ldw<double, W>(A.aE + c, kE);
+    ldw<double, W>(A.aN + c, kN); ldw<double, W>(A.aN + c - A.nI, kS);
+    ldw<double, W>(A.aT + c, kT); ldw<double, W>(A.aT + c - A.nIJ, kB);
+#pragma unroll
+    for (int m = 0; m < W; ++m)
+        y[0][m] = kP[m] * o[m] + kE[m] * (m + 1 < W ? o[m + 1 < W ? m + 1 : 0] : e) + (m ? kE[m ? m - 1 : 0] : kw) * (m ? o[m ? m - 1 : 0] : w)
+                  + kN[m] * n[m] + kS[m] * s[m] + kT[m] * t[m] + kB[m] * b[m];
+#pragma unroll
+    for (int m = 0; m < W; ++m)   // W divides 32: the group's cells share a word
+        if (is_ghost(gw, c + m)) {
+            double g[1];
+            ghost_row<1>(A.gh, ghost_index(gw, c + m), [&](int q, long long e_) { return f.one(q, e_); }, g);
+            y[0][m] = g[0];
+        }
+}
+
+struct BiVecs {
+    double *x, *r, *s, *t, *rp;
+    const double* invD;
+    long long N, PS;
+};
+
+// sweep 1:  x += xa P + xo S;  R = S - omega T;  P' = R + beta (P - omega V);  v = A P';  sums (rp, v)
+template <int NR, int W, class Op>
+__device__ __forceinline__ void bi_sweep1(const Op& A, const BiVecs& b, const double* P, const double* V, double* Pn, double* Vn, const bool (&run)[NR],
+                                          const double (&xa)[NR], const double (&xo)[NR], const double (&omega)[NR], const double (&beta)[NR],
+                                          double (&acc)[NR]) {
+    struct F {
+        const double *S, *Tt, *P, *V;
+        long long PS;
+        const double (&om)[NR], (&be)[NR];
+        __device__ __forceinline__ double one(int q, long long e) const {
+            const long long i = q * PS + e;
+            return (S[i] - om[q] * Tt[i]) + be[q] * (P[i] - om[q] * V[i]);
+        }
+        __device__ __forceinline__ void vec(long long e, double (&o)[W]) const {
+            double s[W], t[W], p[W], v[W];
+            ldw<double, W>(S + e, s); ldw<double, W>(Tt + e, t); ldw<double, W>(P + e, p); ldw<double, W>(V + e, v);
+#pragma unroll
+            for (int m = 0; m < W; ++m) o[m] = (s[m] - om[0] * t[m]) + be[0] * (p[m] - om[0] * v[m]);
+        }
+    } f{b.s, b.t, P, V, b.PS, omega, beta};
+    const long long step = W * (long long)gridDim.x * blockDim.x;
+    for (long long c = W * (blockIdx.x * (long long)blockDim.x + threadIdx.x); c < b.N; c += step) {
+        double y[NR][W], id[W];
+        apply_w<NR, W>(A, c, f, y);
+        ldw<double, W>(b.invD + c, id);
+#pragma unroll
+        for (int q = 0; q < NR; ++q) {
+            if (!run[q]) continue;
+            const long long i = q * b.PS + c;
+            double s[W], t[W], p[W], v[W], x[W], rp[W];
+            ldw<double, W>(b.s + i, s); ldw<double, W>(b.t + i, t); ldw<double, W>(P + i, p); ldw<double, W>(V + i, v);
+            ldw<double, W>(b.x + i, x); ldw<double, W>(b.rp + i, rp);
+#pragma unroll
+            for (int m = 0; m < W; ++m) {
+                x[m] = x[m] + (xa[q] * p[m] + xo[q] * s[m]);
+                s[m] = s[m] - omega[q] * t[m];
+                p[m] = s[m] + beta[q] * (p[m] - omega[q] * v[m]);
+                acc[q] += rp[m] * y[q][m];
+                v[m] = id[m] * y[q][m];
+            }
+            stw<double, W>(b.x + i, x); stw<double, W>(b.r + i, s); stw<double, W>(Pn + i, p); stw<double, W>(Vn + i, v);
+        }
+    }
+}
+
+// sweep 2:  S = R - alpha V;  t = A S;  sums (t, s), (t, t), (rp, s), (rp, t), (s, s)
+template <int NR, int W, class Op>
+__device__ __forceinline__ void bi_sweep2(const Op& A, const BiVecs& b, const double* V, const bool (&run)[NR], const double (&alpha)[NR],
+                                          double (&acc)[5 * NR]) {
+    struct F {
+        const double *R, *V;
+        long long PS;
+        const double (&al)[NR];
+        __device__ __forceinline__ double one(int q, long long e) const { return R[q * PS + e] - al[q] * V[q * PS + e]; }
+        __device__ __forceinline__ void vec(long long e, double (&o)[W]) const {
+            double r[W], v[W];
+            ldw<double, W>(R + e, r); ldw<double, W>(V + e, v);
+#pragma unroll
+            for (int m = 0; m < W; ++m) o[m] = r[m] - al[0] * v[m];
+        }
+    } f{b.r, V, b.PS, alpha};
+    const long long step = W * (long long)gridDim.x * blockDim.x;
+    for (long long c = W * (blockIdx.x * (long long)blockDim.x + threadIdx.x); c < b.N; c += step) {
+        double y[NR][W], id[W];
+        apply_w<NR, W>(A, c, f, y);
+        ldw<double, W>(b.invD + c, id);
+#pragma unroll
+        for (int q = 0; q < NR; ++q) {
+            if (!run[q]) continue;
+            const long long i = q * b.PS + c;
+            double s[W], v[W], rp[W];
+            ldw<double, W>(b.r + i, s); ldw<double, W>(V + i, v); ldw<double, W>(b.rp + i, rp);
+#pragma unroll
+            for (int m = 0; m < W; ++m) {
+                s[m] = s[m] - alpha[q] * v[m];
+                const double d = diag_of(A, c + m), sv = (d != 0. ? d : 1.) * s[m], tv = y[q][m];
+                acc[5 * q] += tv * sv; acc[5 * q + 1] += tv * tv;
+                acc[5 * q + 2] += rp[m] * sv; acc[5 * q + 3] += rp[m] * tv;
+                acc[5 * q + 4] += sv * sv;
+                v[m] = id[m] * y[q][m];
+            }
+            stw<double, W>(b.s + i, s); stw<double, W>(b.t + i, v);
+        }
+    }
+}
+
+// omega, next beta and rho, and (r, r) from the sums of sweep 2
+__device__ __forceinline__ void bi_scalars(const double* t, double alpha, double& omega, double& beta, double& rho, double& rr) {
+    omega = t[1] == 0. ? 0. : t[0] / t[1];
+    const double rn = t[2] - omega * t[3];
+    rr = t[4] - 2. * omega * t[0] + omega * omega * t[1];
+    beta = (rn / rho) * (alpha / omega);
+    rho = rn;
+}
+
+template <int NR, class Op, int W>
+__global__ void __launch_bounds__(W == 2 ? 640 : 512) bicgstab_kernel(Op A, KArgs a) {
+    if (a.skip_if_ok && *a.skip_if_ok == 0) return;   // uniform across the grid: no barrier is reached
+    if (a.skip_if_ok && blockIdx.x == 0 && threadIdx.x == 0 && a.fallbacks) atomicAdd(a.fallbacks, 1);
+    GridRed grid(a.partials);
+    const long long N = a.N, PS = a.PS;
+    const long long T = (long long)gridDim.x * blockDim.x;
+    const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const double* invD = a.invD;
+    if (NR == 1 && a.project) project_mean(grid, const_cast<double*>(a.b), N, t0, T);
+    // ---- initial state: x = 0, r = rp = b (S holds it for the first sweep, with P = V = T = 0)
+    double bb[NR];
+    {
+        double acc[NR];
+#pragma unroll
+        for (int q = 0; q < NR; ++q) acc[q] = 0.;
+        for (long long c = t0; c < N; c += T)
+#pragma unroll
+            for (int q = 0; q < NR; ++q) {
+                const double bv = a.b[q * PS + c];
+                a.x[q * PS + c] = 0.;
+                a.s[q * PS + c] = invD[c] * bv;
+                a.rp[q * PS + c] = bv;
+                a.t[q * PS + c] = 0.; a.p[0][q * PS + c] = 0.; a.v[0][q * PS + c] = 0.;
+                acc[q] += bv * bv;
+            }
+        grid.sum<NR>(acc, bb);
+    }
+    double rho[NR], alpha[NR], omega[NR], beta[NR], tol2[NR], relres[NR];
+    int it[NR], status[NR];
+    bool done[NR];
+#pragma unroll
+    for (int q = 0; q < NR; ++q) {
+        rho[q] = bb[q]; alpha[q] = 0.; omega[q] = 0.; beta[q] = 0.;
+        tol2[q] = fmax(a.rtol * a.rtol * bb[q], a.atol * a.atol);
+        it[q] = 0; relres[q] = 0.;
+        // x = 0 already meets the absolute floor: nothing to do (relative residual 1)
+        done[q] = !(bb[q] > 0.) || bb[q] <= tol2[q];
+        if (bb[q] > 0. && done[q]) relres[q] = 1.;
+        status[q] = bb[q] != bb[q] ? 3 : 0;
+    }
+    BiVecs v;
+    v.x = a.x; v.r = a.r; v.s = a.s; v.t = a.t; v.rp = a.rp; v.invD = invD; v.N = N; v.PS = PS;
+    int cur = 0;
+    while (true) {
+        bool run[NR], needT[NR], any = false;
+#pragma unroll
+        for (int q = 0; q < NR; ++q) { run[q] = !done[q]; any |= run[q]; needT[q] = false; }
+        if (!any) break;
+        // ---- sweep 1
+        {
+            double acc[NR], rv[NR];
+#pragma unroll
+            for (int q = 0; q < NR; ++q) acc[q] = 0.;
+            bi_sweep1<NR, W>(A, v, a.p[cur], a.v[cur], a.p[cur ^ 1], a.v[cur ^ 1], run, alpha, omega, omega, beta, acc);
+            grid.sum<NR>(acc, rv);
+#pragma unroll
+            for (int q = 0; q < NR; ++q) {
+                alpha[q] = omega[q] = 0.;   // x is up to date with R
+                if (!run[q]) continue;
+                if (rv[q] == 0. || rv[q] != rv[q]) { needT[q] = true; run[q] = false; }
+                else alpha[q] = rho[q] / rv[q];
+            }
+        }
+        cur ^= 1;
+        // ---- sweep 2
+        {
+            double acc[5 * NR], tot[5 * NR];
+#pragma unroll
+            for (int q = 0; q < 5 * NR; ++q) acc[q] = 0.;
+            bi_sweep2<NR, W>(A, v, a.v[cur], run, alpha, acc);
+            grid.sum<5 * NR>(acc, tot);
+            bool anyT = false;
+#pragma unroll
+            for (int q = 0; q < NR; ++q) {
+                if (run[q]) {
+                    double rr;
+                    it[q] += 1;
+                    bi_scalars(tot + 5 * q, alpha[q], omega[q], beta[q], rho[q], rr);
+                    if (rr <= tol2[q] || omega[q] == 0. || it[q] >= a.maxit || rr != rr) needT[q] = true;
+                }
+                anyT |= needT[q];
+            }
+            if (!anyT) continue;
+        }
+        // ---- true residual r = b - A x of the right-hand sides being checked
+        for (long long c = t0; c < N; c += T)
+#pragma unroll
+            for (int q = 0; q < NR; ++q) {
+                const long long i = q * PS + c;
+                if (needT[q]) a.x[i] = a.x[i] + (alpha[q] * a.p[cur][i] + omega[q] * a.s[i]);
+            }
+        grid.sync();
+        double acc[NR], rrT[NR];
+#pragma unroll
+        for (int q = 0; q < NR; ++q) acc[q] = 0.;
+        for (long long c = t0; c < N; c += T) {
+            double y[NR];
+            apply<NR>(A, c, [&](int q, long long e) { return a.x[q * PS + e]; }, y);
+#pragma unroll
+            for (int q = 0; q < NR; ++q) {
+                if (!needT[q]) continue;
+                const long long i = q * PS + c;
+                const double rt = a.b[i] - y[q];
+                a.s[i] = invD[c] * rt; a.rp[i] = rt;
+                a.t[i] = 0.; a.p[cur][i] = 0.; a.v[cur][i] = 0.;
+                acc[q] += rt * rt;
+            }
+        }
+        grid.sum<NR>(acc, rrT);
+#pragma unroll
+        for (int q = 0; q < NR; ++q) {
+            if (!needT[q]) continue;
+            relres[q] = sqrt(rrT[q] / bb[q]);
+            if (rrT[q] <= tol2[q]) { done[q] = true; status[q] = 0; }
+            else if (rrT[q] != rrT[q]) { done[q] = true; status[q] = 3; }
+            else if (it[q] >= a.maxit) { done[q] = true; status[q] = 1; }
+            else { rho[q] = rrT[q]; alpha[q] = omega[q] = beta[q] = 0.; }   // restart from the true residual
+        }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        for (int q = 0; q < NR; ++q) { a.out->iters[q] = it[q]; a.out->relres[q] = relres[q]; a.out->status[q] = status[q]; }
+    }
+}
+
+// ------------------------------------------------------------------ BiCGStab, three right-hand sides
+// The momentum solve: three right-hand sides share one operator sweep.  Classic order of the method,
+// three sweeps and reductions per iteration: with three right-hand sides the two-sweep form needs 15
+// sums and twelve vectors at the stencil neighbours, spills at 128 registers and takes the same time
+// (0.36 against 0.38 ms per iteration at 128^3), and a solve is 3 to 15 iterations.  Two blocks of KB
+// threads per SM, partials summed in block order.
 constexpr int KB = 256;   // threads per block
 constexpr int KP = 8;     // partial slots per block
-
-__device__ __forceinline__ double ldcg(const double* p) { return *p; }   // coherent load after a grid barrier
 
 template <int K>
 __device__ __forceinline__ void warp_sum(double (&v)[K]) {
@@ -105,7 +476,7 @@ __device__ void grid_totals(const double* partials, double (&out)[K]) {
 // that races ahead to the next reduction cannot overwrite a slot another block is still
 // summing, because it must first pass the barrier of the reduction in between.
 template <int K>
-__device__ __forceinline__ void grid_reduce(cg::grid_group& grid, double (&v)[K], double* partials, int& parity, double (&out)[K]) {
+__device__ __forceinline__ void grid_reduce(GridRed& grid, double (&v)[K], double* partials, int& parity, double (&out)[K]) {
     double* buf = partials + (long long)(parity & 1) * gridDim.x * KP;
     block_partials<K>(v, buf);
     grid.sync();
@@ -113,57 +484,9 @@ __device__ __forceinline__ void grid_reduce(cg::grid_group& grid, double (&v)[K]
     ++parity;
 }
 
-
-template <class Op>
-__global__ void inv_diag_kernel(Op A, long long N, double* invD) {
-    long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (c >= N) return;
-    double dg = diag_of(A, c);
-    invD[c] = dg != 0. ? 1. / dg : 1.;
-}
-
-struct KArgs {
-    const double* b;
-    double* x;
-    double* r;
-    double* rp;
-    double* p[2];
-    double* v[2];
-    double* t;
-    const double* invD;
-    double* partials;
-    KspOut* out;
-    long long N, PS;
-    double rtol;
-    double atol;   // absolute floor: converged when ||b - A x|| <= max(rtol ||b||, atol)
-    int maxit;
-    int project;   // remove the mean of b first (singular all-Neumann pressure systems)
-    // fallback mode: when skip_if_ok is set the launch returns at once unless the status
-    // it points to (the previous solve's) is non-zero; fallbacks counts the launches that ran
-    const int* skip_if_ok;
-    int* fallbacks;
-};
-
-// Remove the mean of b (one plane), in place; every block computes the same mean.
-__device__ __forceinline__ void project_mean(cg::grid_group& grid, double* b, long long N, long long t0, long long T,
-                                             double* partials, int& par) {
-    double s[1] = {0.};
-    for (long long c = t0; c < N; c += T) s[0] += b[c];
-    double tot[1];
-    grid_reduce<1>(grid, s, partials, par, tot);
-    double mean = tot[0] / (double)N;
-    for (long long c = t0; c < N; c += T) b[c] = b[c] - mean;
-    // the projected b is read at stencil neighbours owned by other blocks right after this
-    // (CG forms w = A D^-1 b): every block's subtraction must be visible first
-    grid.sync();
-}
-
-// ------------------------------------------------------------------ BiCGStab
 template <int NR, class Op>
-__global__ void __launch_bounds__(KB) bicgstab_kernel(Op A, KArgs a) {
-    if (a.skip_if_ok && *a.skip_if_ok == 0) return;   // uniform across the grid: no barrier is reached
-    if (a.skip_if_ok && blockIdx.x == 0 && threadIdx.x == 0 && a.fallbacks) atomicAdd(a.fallbacks, 1);
-    cg::grid_group grid = cg::this_grid();
+__global__ void __launch_bounds__(KB, 2) bicgstab3_kernel(Op A, KArgs a) {
+    GridRed grid(a.partials);
     const long long N = a.N, PS = a.PS;
     const long long T = (long long)gridDim.x * blockDim.x;
     const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -171,7 +494,6 @@ __global__ void __launch_bounds__(KB) bicgstab_kernel(Op A, KArgs a) {
 
     double acc[2 * NR];
     int par = 0;
-    if (NR == 1 && a.project) project_mean(grid, const_cast<double*>(a.b), N, t0, T, a.partials, par);
     // ---- initial state: x = 0, r = rp = b
 #pragma unroll
     for (int q = 0; q < NR; ++q) acc[q] = 0.;
@@ -190,7 +512,7 @@ __global__ void __launch_bounds__(KB) bicgstab_kernel(Op A, KArgs a) {
         double tmp[NR];
 #pragma unroll
         for (int q = 0; q < NR; ++q) tmp[q] = acc[q];
-        grid_reduce<NR>(grid, tmp, a.partials, par, bb);
+        grid_reduce<NR>(grid, tmp, a.partials + 16, par, bb);
     }
 
     double rho[NR], rho_old[NR], alpha[NR], omega[NR], tol2[NR];
@@ -248,7 +570,7 @@ __global__ void __launch_bounds__(KB) bicgstab_kernel(Op A, KArgs a) {
             double tmp[NR];
 #pragma unroll
             for (int q = 0; q < NR; ++q) tmp[q] = acc[q];
-            grid_reduce<NR>(grid, tmp, a.partials, par, rv);
+            grid_reduce<NR>(grid, tmp, a.partials + 16, par, rv);
         }
 #pragma unroll
         for (int q = 0; q < NR; ++q) {
@@ -278,7 +600,7 @@ __global__ void __launch_bounds__(KB) bicgstab_kernel(Op A, KArgs a) {
             double tmp[2 * NR];
 #pragma unroll
             for (int q = 0; q < 2 * NR; ++q) tmp[q] = acc[q];
-            grid_reduce<2 * NR>(grid, tmp, a.partials, par, tot);
+            grid_reduce<2 * NR>(grid, tmp, a.partials + 16, par, tot);
         }
 #pragma unroll
         for (int q = 0; q < NR; ++q) {
@@ -307,7 +629,7 @@ __global__ void __launch_bounds__(KB) bicgstab_kernel(Op A, KArgs a) {
             double tmp[2 * NR];
 #pragma unroll
             for (int q = 0; q < 2 * NR; ++q) tmp[q] = acc[q];
-            grid_reduce<2 * NR>(grid, tmp, a.partials, par, tot);
+            grid_reduce<2 * NR>(grid, tmp, a.partials + 16, par, tot);
         }
         bool anyT = false;
 #pragma unroll
@@ -343,7 +665,7 @@ __global__ void __launch_bounds__(KB) bicgstab_kernel(Op A, KArgs a) {
                 double tmp[NR];
 #pragma unroll
                 for (int q = 0; q < NR; ++q) tmp[q] = acc[q];
-                grid_reduce<NR>(grid, tmp, a.partials, par, rrT);
+                grid_reduce<NR>(grid, tmp, a.partials + 16, par, rrT);
             }
 #pragma unroll
             for (int q = 0; q < NR; ++q) {
@@ -373,10 +695,11 @@ __global__ void __launch_bounds__(KB) bicgstab_kernel(Op A, KArgs a) {
 // u_{i+1} at the stencil neighbours is recomputed from r_i, w_i and s_{i-1}, which are
 // double-buffered (the sweep writes the other buffer).
 template <class Op>
-__global__ void __launch_bounds__(KB, 4) cg1_kernel(Op A, KArgs a) {
+__global__ void __launch_bounds__(1024) cg1_kernel(Op A, KArgs a) {
     if (a.skip_if_ok && *a.skip_if_ok == 0) return;   // uniform across the grid: no barrier is reached
+    if (a.cs[0] && scaled_form(a.out)) return;        // cgs_kernel ran
     if (a.skip_if_ok && blockIdx.x == 0 && threadIdx.x == 0 && a.fallbacks) atomicAdd(a.fallbacks, 1);
-    cg::grid_group grid = cg::this_grid();
+    GridRed grid(a.partials);
     const long long N = a.N, PS = a.PS;
     const long long T = (long long)gridDim.x * blockDim.x;
     const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -384,8 +707,7 @@ __global__ void __launch_bounds__(KB, 4) cg1_kernel(Op A, KArgs a) {
     // current (read) and next (written) buffers, swapped after every sweep
     double *rC = a.r, *rN = a.r + PS, *wC = a.v[0], *wN = a.v[1], *sC = a.p[0], *sN = a.p[1];
     double* p = a.t;       // u = M^-1 r is not stored: it is recomputed from r where needed
-    int par = 0;
-    if (a.project) project_mean(grid, const_cast<double*>(a.b), N, t0, T, a.partials, par);
+    if (a.project) project_mean(grid, const_cast<double*>(a.b), N, t0, T);
     // ---- start: x = 0, r = b, u = M^-1 b, w = A u, s_-1 = p_-1 = 0
     double acc[3] = {0., 0., 0.};
     for (long long c = t0; c < N; c += T) {
@@ -398,7 +720,7 @@ __global__ void __launch_bounds__(KB, 4) cg1_kernel(Op A, KArgs a) {
         acc[0] += bv * uv; acc[1] += y[0] * uv; acc[2] += bv * bv;
     }
     double tot[3];
-    grid_reduce<3>(grid, acc, a.partials, par, tot);
+    grid.sum<3>(acc, tot);
     double gamma = tot[0], bb = tot[2];
     double tol2 = fmax(a.rtol * a.rtol * bb, a.atol * a.atol);
     double alpha = tot[1] != 0. ? gamma / tot[1] : 0., beta = 0.;
@@ -430,7 +752,7 @@ __global__ void __launch_bounds__(KB, 4) cg1_kernel(Op A, KArgs a) {
             s1[c] = si; p[c] = pi; r1[c] = rn; w1[c] = y[0];
             acc[0] += rn * un; acc[1] += y[0] * un; acc[2] += rn * rn;
         }
-        grid_reduce<3>(grid, acc, a.partials, par, tot);
+        grid.sum<3>(acc, tot);
         it += 1;
         { double* t_ = rC; rC = rN; rN = t_; t_ = wC; wC = wN; wN = t_; t_ = sC; sC = sN; sN = t_; }
         double gn = tot[0], dn = tot[1], rr = tot[2];
@@ -451,7 +773,7 @@ __global__ void __launch_bounds__(KB, 4) cg1_kernel(Op A, KArgs a) {
                 a2[0] += rt * rt;
             }
             double t1[1];
-            grid_reduce<1>(grid, a2, a.partials, par, t1);
+            grid.sum<1>(a2, t1);
             relres = sqrt(t1[0] / bb);
             if (t1[0] <= tol2) { done = true; status = 0; }
             else if (t1[0] != t1[0]) { done = true; status = 3; }
@@ -469,7 +791,7 @@ __global__ void __launch_bounds__(KB, 4) cg1_kernel(Op A, KArgs a) {
                     a3[0] += rc[c] * uv; a3[1] += y[0] * uv;
                 }
                 double t2[2];
-                grid_reduce<2>(grid, a3, a.partials, par, t2);
+                grid.sum<2>(a3, t2);
                 gamma = t2[0];
                 alpha = t2[1] != 0. ? gamma / t2[1] : 0.;
                 beta = 0.;
@@ -480,235 +802,214 @@ __global__ void __launch_bounds__(KB, 4) cg1_kernel(Op A, KArgs a) {
     if (blockIdx.x == 0 && threadIdx.x == 0) { a.out->iters[0] = it; a.out->relres[0] = relres; a.out->status[0] = status; }
 }
 
-// ------------------------------------------------------------------ mixed precision
-// FP64 iterative refinement around FP32 inner solves (the precision form of the pressure
-// correction): the true residual r = b - A x, the update x += e, and every dot product and
-// norm stay FP64; the matrix copy, the Jacobi preconditioner, the inner Krylov vectors and
-// the inner operator sweeps are FP32.  One launch runs the whole solve:
-//   repeat: r = b - A x (FP64, reduced) -> stop at ||r|| <= rtol ||b||;
-//           A32 e = float(r) by FP32 CG or BiCGStab to inner_rtol (relative);  x += e.
-struct OpSymF {
-    const float* aP;
-    const float* aE;
-    const float* aN;
-    const float* aT;
-    long long nI, nIJ;
-    GhostRows gh;
-};
-
-template <class X>
-__device__ __forceinline__ float applyf(const OpSymF& A, long long c, X&& x) {
-    float aP = __ldg(A.aP + c), aE = __ldg(A.aE + c), aW = __ldg(A.aE + c - 1), aN = __ldg(A.aN + c);
-    float aS = __ldg(A.aN + c - A.nI), aT = __ldg(A.aT + c), aB = __ldg(A.aT + c - A.nIJ);
-    float y = aP * x(c) + aE * x(c + 1) + aW * x(c - 1) + aN * x(c + A.nI) + aS * x(c - A.nI) + aT * x(c + A.nIJ)
-              + aB * x(c - A.nIJ);
-    if (A.gh.n > 0) {
-        uint32_t wbits = __ldg(A.gh.bits + (c >> 5));
-        if ((wbits >> (c & 31)) & 1u) {
-            int g = ghost_index(A.gh, c);
-            float sum = 0.f;
-            for (int m = 0; m < 9; ++m) {
-                int col = __ldg(A.gh.col + 9 * g + m);
-                if (col >= 0) sum += (float)__ldg(A.gh.val + 9 * g + m) * x((long long)col);
-            }
-            y = sum;
+// ------------------------------------------------------------------ CG, scaled form
+// The solve's frame around cg_update and cg_product: start, true-residual check, restart and unscaling as in
+// cg1_kernel, which runs instead where the scaled form does not apply.
+template <class Op, int W>
+__global__ void __launch_bounds__(1024) cgs_kernel(Op A, KArgs a) {
+    if (a.skip_if_ok && *a.skip_if_ok == 0) return;
+    if (!scaled_form(a.out)) return;
+    if (a.skip_if_ok && blockIdx.x == 0 && threadIdx.x == 0 && a.fallbacks) atomicAdd(a.fallbacks, 1);
+    GridRed grid(a.partials);
+    const long long N = a.N;
+    const long long T = (long long)gridDim.x * blockDim.x;
+    const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const double* S = a.invD;
+    const double sg = diag_of(A, 0) > 0. ? 1. : -1.;
+    CgVecs<double> v;
+    v.r = a.r; v.q = a.v[0]; v.p = a.p[0]; v.y = a.x;
+    v.E = a.cs[0]; v.N = a.cs[1]; v.U = a.cs[2];
+    v.d = diag_plane(A);
+    v.n = (int)N; v.nI = (int)A.nI; v.nIJ = (int)A.nIJ;
+    if (a.project) project_mean(grid, const_cast<double*>(a.b), N, t0, T);
+    double bb;
+    {
+        double s[1] = {0.}, tot[1];
+        for (long long c = t0; c < N; c += T) {
+            const double bv = a.b[c];
+            v.r[c] = sg * S[c] * bv; v.q[c] = 0.; v.p[c] = 0.; v.y[c] = 0.;
+            s[0] += bv * bv;
         }
+        grid.sum<1>(s, tot);
+        bb = tot[0];
     }
-    return y;
+    const double tol2 = fmax(a.rtol * a.rtol * bb, a.atol * a.atol);
+    int it = 0, status = 0;
+    double relres = 0.;
+    bool done = !(bb > 0.) || bb <= tol2;   // x = 0 already meets the absolute floor
+    if (bb > 0. && done) relres = 1.;
+    if (bb != bb) status = 3;
+    double alpha = 0., beta = 0., best = bb;
+    bool first = true;                      // the first update forms p = r only
+    while (!done) {
+        double acc[4] = {0., 0., 0., 0.}, tot[4];
+        cg_update<double, W>(v, alpha, beta, false, acc[0], acc[1]);
+        grid.sync();
+        cg_product<double, W>(v, true, acc[2], acc[3]);
+        grid.sum<4>(acc, tot);
+        if (!first) ++it;
+        const bool broke = !cg_scalars(tot[0], tot[2], tot[3], alpha, beta);
+        const bool stuck = broke && first;   // no direction from a fresh residual: a restart would not help
+        if (tot[1] < best) best = tot[1];
+        if ((!first && (tot[1] <= tol2 || it >= a.maxit)) || !(tot[1] <= 1e6 * best) || broke) {
+            // ---- true residual r = b - A x, x = S y
+            double s[3] = {0., 0., 0.}, t[3];
+            for (long long c = t0; c < N; c += T) {
+                double y[1];
+                apply<1>(A, c, [&](int, long long e) { return S[e] * v.y[e]; }, y);
+                const double rt = a.b[c] - y[0], rs = sg * S[c] * rt;
+                v.r[c] = rs; v.q[c] = 0.; v.p[c] = 0.;
+                s[0] += rt * rt; s[1] += rs * rs; s[2] += rt;
+            }
+            grid.sum<3>(s, t);
+            relres = sqrt(t[0] / bb);
+            if (t[0] <= tol2) { done = true; status = 0; }
+            else if (t[0] != t[0]) { done = true; status = 3; }
+            else if (it >= a.maxit) { done = true; status = 1; }
+            else if (stuck || t[1] == 0.) { done = true; status = 2; }
+            alpha = beta = 0.;   // restart from the true residual, in the range of a singular A
+            first = true;
+            best = t[0];
+            if (a.project)
+                for (long long c = t0; c < N; c += T) v.r[c] = v.r[c] - sg * S[c] * (t[2] / (double)N);
+        } else
+            first = false;
+    }
+    for (long long c = t0; c < N; c += T) a.x[c] = S[c] * v.y[c];
+    if (blockIdx.x == 0 && threadIdx.x == 0) { a.out->iters[0] = it; a.out->relres[0] = relres; a.out->status[0] = status; }
 }
 
-__global__ void cast_sym_kernel(OpSym A, long long N, float* aP, float* aE, float* aN, float* aT, float* invD) {
+// ------------------------------------------------------------------ mixed precision
+// FP32 CG inside FP64 iterative refinement (the precision form of the pressure correction): the
+// true residual r = b - A x, the update x += e, and every dot product and norm stay FP64; the scaled
+// operator's planes, the Krylov vectors and the operator sweeps are FP32.  One launch runs the whole
+// solve.
+//
+// A refinement does not restart the Krylov process (Sleijpen & van der Vorst 1996, reliable
+// updates): whenever the recursive residual has fallen by MX_DROP since the last one, x takes the
+// FP32 correction, the FP64 residual replaces the recursive one, and the iteration goes on with the
+// search direction it has.  Restarting instead cost the 128^3 skewed cavity 1950 iterations a
+// step against 1680, as many as in FP64.  A recursive residual that has left the true one, or
+// MX_PATIENCE iterations without a new smallest residual, count as a stall: the process restarts from
+// the true residual, and the second stall in a row leaves the solve to the FP64 fallback.
+//
+// Symmetric systems only.  With immersed-boundary ghost rows the mixed form runs the FP64 BiCGStab: FP32
+// BiCGStab loses its biorthogonality there.  Measured on 72x48x48 and 75x39x41 sphere cases (FP64
+// 4719 and 5690 iterations a step, 66 and 76 ms): FP32 to 1e-6 and restarted, stalled in every
+// solve, then the FP64 solve, 0.5-1.2 s; FP32 with reliable updates 24829 and 23281 iterations, 547
+// and 266 ms; FP64 vectors on the FP32 matrix 12772 and 10529, 171 and 160 ms.
+constexpr double MX_DROP = 0.05;
+constexpr int MX_PATIENCE = 1000;
+
+__global__ void cast_kernel(long long N, const double* d, float* f) {
     long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (c >= N) return;
-    double d = A.aP[c];
-    aP[c] = (float)d; aE[c] = (float)A.aE[c]; aN[c] = (float)A.aN[c]; aT[c] = (float)A.aT[c];
-    invD[c] = d != 0. ? (float)(1. / d) : 1.f;
+    if (c < N) f[c] = (float)d[c];
 }
 
 struct MxArgs {
     const double* b;
     double* x;
-    float* r[2];
-    float* w[2];
-    float* s[2];
-    float* p;
-    float* e;
-    float* v[2];
-    float* t;
-    const float* invD;
+    float *r, *q, *p, *e;
+    const float* d;         // the diagonal
+    const float* cs[3];     // the scaled operator's planes
+    const double* S;        // 1 / sqrt|d|
     double* partials;
     KspOut* out;
     long long N;
     double rtol;
     double atol;
     int maxit;
-    double eta;
     int project;
-    int inner_max;
 };
 
-template <class Op64, int INNER_BICG>
-__global__ void __launch_bounds__(KB, 4) mixed_kernel(Op64 A, OpSymF Af, MxArgs a) {
-    cg::grid_group grid = cg::this_grid();
-    const long long N = a.N;
-    const long long T = (long long)gridDim.x * blockDim.x;
-    const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const float* invD = a.invD;
-    int par = 0;
-    if (a.project) project_mean(grid, const_cast<double*>(a.b), N, t0, T, a.partials, par);
-    double acc1[1] = {0.};
-    for (long long c = t0; c < N; c += T) {
-        double bv = a.b[c];
-        a.x[c] = 0.;
-        acc1[0] += bv * bv;
+// Watches the residual norms.
+struct MxWatch {
+    double tol2, best, top;      // ||r||^2: tolerance, smallest so far, largest since the last refinement
+    int since = 0, stalls = 0;   // iterations since the smallest, stalls in a row
+    __device__ void start(double rr) { best = top = rr; }
+    // after an iteration: whether to refine now
+    __device__ bool due(double rr) {
+        if (rr < best) { best = rr; since = 0; stalls = 0; } else ++since;
+        if (rr > top) top = rr;
+        return rr <= tol2 || rr <= MX_DROP * MX_DROP * top || since >= MX_PATIENCE || rr != rr;
     }
-    double tot1[1];
-    grid_reduce<1>(grid, acc1, a.partials, par, tot1);
-    double bb = tot1[0], tol2 = fmax(a.rtol * a.rtol * bb, a.atol * a.atol);
-    int status = 0, inner_total = 0, outer = 0;
-    double relres = 0.;
-    bool done = !(bb > 0.);
-    if (bb != bb) { status = 3; done = true; }
-    float* rC = a.r[0];
-    float* rN = a.r[1];
-    while (!done) {
-        // ---- FP64 true residual, handed to the inner solver in FP32
-        acc1[0] = 0.;
+    // at a refinement from the recursive rr to the true one: whether the process has to restart
+    __device__ bool refine(double rr, double truth) {
+        const bool stalled = since >= MX_PATIENCE || !(fabs(rr) > 0.25 * truth && fabs(rr) < 4. * truth);
+        if (stalled) { ++stalls; since = 0; best = truth; }
+        top = truth;
+        return stalled;
+    }
+};
+
+template <int W>
+__global__ void __launch_bounds__(1024) mixed_cg_kernel(OpSym A, MxArgs a) {
+    GridRed grid(a.partials);
+    const long long N = a.N, T = (long long)gridDim.x * blockDim.x, t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const double sg = diag_of(A, 0) > 0. ? 1. : -1.;
+    CgVecs<float> v;
+    v.r = a.r; v.q = a.q; v.p = a.p; v.y = a.e;
+    v.E = a.cs[0]; v.N = a.cs[1]; v.U = a.cs[2]; v.d = a.d;
+    v.n = (int)N; v.nI = (int)A.nI; v.nIJ = (int)A.nIJ;
+    if (a.project) project_mean(grid, const_cast<double*>(a.b), N, t0, T);
+    double bb;
+    {
+        double s[1] = {0.}, t[1];
         for (long long c = t0; c < N; c += T) {
-            double y[1];
-            apply<1>(A, c, [&](int, long long e_) { return a.x[e_]; }, y);
-            double rt = a.b[c] - y[0];
-            rC[c] = (float)rt;
-            acc1[0] += rt * rt;
+            const double bv = a.b[c], rs = sg * a.S[c] * bv;
+            v.r[c] = (float)rs; v.q[c] = 0.f; v.p[c] = 0.f; v.y[c] = 0.f;
+            a.x[c] = 0.;
+            s[0] += bv * bv;
         }
-        grid_reduce<1>(grid, acc1, a.partials, par, tot1);
-        double rr = tot1[0];
-        relres = sqrt(rr / bb);
-        if (rr <= tol2) { status = 0; break; }
-        if (rr != rr) { status = 3; break; }
-        if (inner_total >= a.maxit) { status = 1; break; }
-        ++outer;
-        // inner target: as deep as FP32 allows on the first pass, then only the factor still
-        // missing to the outer tolerance (with a safety margin)
-        double eta = 0.25 * sqrt(tol2 / rr);
-        if (eta < a.eta) eta = a.eta;
-        if (eta > 0.5) eta = 0.5;
-        // ---- FP32 inner solve A32 e = r (e from zero), dots and norms in FP64
-        int inner = 0;
-        if (!INNER_BICG) {
-            // Chronopoulos-Gear CG, as cg1_kernel, in FP32 storage
-            float* wC = a.w[0]; float* wN = a.w[1]; float* sC = a.s[0]; float* sN = a.s[1];
-            double acc[3] = {0., 0., 0.};
-            for (long long c = t0; c < N; c += T) {
-                float r0 = rC[c];
-                float u0 = __ldg(invD + c) * r0;
-                float y = applyf(Af, c, [&](long long e_) { return __ldg(invD + e_) * rC[e_]; });
-                a.e[c] = 0.f; wC[c] = y; sC[c] = 0.f; a.p[c] = 0.f;
-                acc[0] += (double)r0 * u0; acc[1] += (double)y * u0; acc[2] += (double)r0 * r0;
-            }
-            double tot[3];
-            grid_reduce<3>(grid, acc, a.partials, par, tot);
-            double gamma = tot[0], rr0 = tot[2];
-            double alpha = tot[1] != 0. ? gamma / tot[1] : 0., beta = 0.;
-            double tin2 = eta * eta * rr0;
-            bool stop = !(gamma != 0.);
-            while (!stop) {
-                float al = (float)alpha, be = (float)beta;
-                acc[0] = acc[1] = acc[2] = 0.;
-                for (long long c = t0; c < N; c += T) {
-                    float idc = __ldg(invD + c);
-                    float r0 = rC[c];
-                    float si = wC[c] + be * sC[c];
-                    float pi = idc * r0 + be * a.p[c];
-                    a.e[c] = a.e[c] + al * pi;
-                    float rn = r0 - al * si;
-                    float un = idc * rn;
-                    float y = applyf(Af, c, [&](long long e_) { return __ldg(invD + e_) * (rC[e_] - al * (wC[e_] + be * sC[e_])); });
-                    sN[c] = si; a.p[c] = pi; rN[c] = rn; wN[c] = y;
-                    acc[0] += (double)rn * un; acc[1] += (double)y * un; acc[2] += (double)rn * rn;
-                }
-                grid_reduce<3>(grid, acc, a.partials, par, tot);
-                ++inner;
-                { float* t_ = rC; rC = rN; rN = t_; t_ = wC; wC = wN; wN = t_; t_ = sC; sC = sN; sN = t_; }
-                double gn = tot[0], dn = tot[1], rri = tot[2];
-                double bn = gn / gamma;
-                double den = dn - bn * gn / alpha;
-                if (rri <= tin2 || inner >= a.inner_max || inner_total + inner >= a.maxit || den == 0. || den != den || gn == 0.) stop = true;
-                beta = bn; alpha = gn / den; gamma = gn;
-            }
-        } else {
-            // BiCGStab, right-preconditioned with Jacobi, in FP32 storage
-            float* rp = a.s[0];
-            float* pO = a.p;  float* pNn = a.s[1];
-            float* vO = a.v[0]; float* vNn = a.v[1];
-            double acc[1] = {0.};
-            for (long long c = t0; c < N; c += T) {
-                float r0 = rC[c];
-                a.e[c] = 0.f; rp[c] = r0; pO[c] = 0.f; vO[c] = 0.f;
-                acc[0] += (double)r0 * r0;
-            }
-            double tot[1];
-            grid_reduce<1>(grid, acc, a.partials, par, tot);
-            double rr0 = tot[0], tin2 = eta * eta * rr0;
-            double rho = rr0, rho_old = 1., alpha = 1., omega = 1.;
-            bool fresh = true, stop = !(rr0 > 0.);
-            float* rcur = rC;
-            while (!stop) {
-                double beta = fresh ? 0. : (rho / rho_old) * (alpha / omega);
-                float be = (float)beta, om = (float)omega;
-                double a1[1] = {0.};
-                for (long long c = t0; c < N; c += T) {
-                    auto pn_at = [&](long long e_) -> float {
-                        float rv = rcur[e_];
-                        return fresh ? rv : rv + be * (pO[e_] - om * vO[e_]);
-                    };
-                    float y = applyf(Af, c, [&](long long e_) { return __ldg(invD + e_) * pn_at(e_); });
-                    pNn[c] = pn_at(c); vNn[c] = y;
-                    a1[0] += (double)rp[c] * y;
-                }
-                double t1[1];
-                grid_reduce<1>(grid, a1, a.partials, par, t1);
-                if (t1[0] == 0. || t1[0] != t1[0]) break;
-                alpha = rho / t1[0];
-                float al = (float)alpha;
-                double a2[2] = {0., 0.};
-                for (long long c = t0; c < N; c += T) {
-                    float y = applyf(Af, c, [&](long long e_) { return __ldg(invD + e_) * (rcur[e_] - al * vNn[e_]); });
-                    float sv = rcur[c] - al * vNn[c];
-                    a.t[c] = y;
-                    a2[0] += (double)y * sv; a2[1] += (double)y * y;
-                }
-                double t2[2];
-                grid_reduce<2>(grid, a2, a.partials, par, t2);
-                omega = t2[1] == 0. ? 0. : t2[0] / t2[1];
-                om = (float)omega;
-                double a3[2] = {0., 0.};
-                for (long long c = t0; c < N; c += T) {
-                    float idc = __ldg(invD + c);
-                    float sv = rcur[c] - al * vNn[c];
-                    a.e[c] = a.e[c] + (al * (idc * pNn[c]) + om * (idc * sv));
-                    float rn = sv - om * a.t[c];
-                    rcur[c] = rn;
-                    a3[0] += (double)rn * rp[c]; a3[1] += (double)rn * rn;
-                }
-                double t3[2];
-                grid_reduce<2>(grid, a3, a.partials, par, t3);
-                ++inner;
-                fresh = false;
-                rho_old = rho; rho = t3[0];
-                { float* t_ = pO; pO = pNn; pNn = t_; t_ = vO; vO = vNn; vNn = t_; }
-                if (t3[1] <= tin2 || omega == 0. || inner >= a.inner_max || inner_total + inner >= a.maxit || t3[1] != t3[1]) stop = true;
-            }
-            rC = rcur;
-        }
-        inner_total += inner;
-        // ---- x += e (FP64); the next residual reads x at the neighbours
-        for (long long c = t0; c < N; c += T) a.x[c] = a.x[c] + (double)a.e[c];
+        grid.sum<1>(s, t);
+        bb = t[0];
+    }
+    MxWatch watch;
+    watch.tol2 = fmax(a.rtol * a.rtol * bb, a.atol * a.atol);
+    watch.start(bb);
+    int it = 0, outer = 0, status = 0;
+    double relres = bb > 0. ? 1. : 0., alpha = 0., beta = 0.;
+    bool done = !(bb > 0.) || bb <= watch.tol2;
+    if (bb != bb) status = 3;
+    if (!scaled_form(a.out)) { done = true; status = 2; }   // not a definite symmetric system: the FP64 solve takes it
+    bool fresh = true;   // the next update forms p = r + beta p only
+    while (!done) {
+        double acc[4] = {0., 0., 0., 0.}, tot[4];
+        cg_update<float, W>(v, (float)alpha, (float)beta, false, acc[0], acc[1]);
         grid.sync();
-        if (outer > 60) { status = 1; break; }
+        cg_product<float, W>(v, true, acc[2], acc[3]);
+        grid.sum<4>(acc, tot);
+        if (!fresh) ++it;
+        const bool broke = !cg_scalars(tot[0], tot[2], tot[3], alpha, beta), stuck = broke && fresh;
+        const bool due = (!fresh && watch.due(tot[1])) || tot[1] != tot[1];
+        fresh = false;
+        if (due || broke || it >= a.maxit) {
+            // ---- x += S y; FP64 true residual in the place of the recursive one; p and q stay
+            for (long long c = t0; c < N; c += T) { a.x[c] = a.x[c] + a.S[c] * (double)v.y[c]; v.y[c] = 0.f; }
+            grid.sync();
+            double s[2] = {0., 0.}, t[2];
+            for (long long c = t0; c < N; c += T) {
+                double y[1];
+                apply<1>(A, c, [&](int, long long e) { return a.x[e]; }, y);
+                const double rt = a.b[c] - y[0], rs = sg * a.S[c] * rt;
+                v.r[c] = (float)rs;
+                s[0] += rt * rt; s[1] += rs * rs;
+            }
+            grid.sum<2>(s, t);
+            ++outer;
+            relres = sqrt(t[0] / bb);
+            if (t[0] <= watch.tol2) { done = true; status = 0; }
+            else if (t[0] != t[0]) { done = true; status = 3; }
+            else if (it >= a.maxit) { done = true; status = 1; }
+            else {
+                const bool restart = watch.refine(tot[1], t[0]) || broke;
+                if (watch.stalls >= 2 || stuck) { done = true; status = 2; }
+                if (restart || !cg_scalars(t[1], tot[2], tot[3], alpha, beta)) { alpha = beta = 0.; fresh = true; }
+            }
+        }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        a.out->iters[0] = inner_total; a.out->iters[1] = outer; a.out->relres[0] = relres; a.out->status[0] = status;
+        a.out->iters[0] = it; a.out->iters[1] = outer; a.out->relres[0] = relres; a.out->status[0] = status;
     }
 }
 
@@ -724,154 +1025,149 @@ static int sm_count() {
     return g_numSM;
 }
 
-template <class K>
-static int coop_grid(K kernel) {
-    int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, KB, 0) != cudaSuccess || nb < 1) nb = 1;
-    if (nb > 4) nb = 4;
-    return nb * sm_count();
+// Shape of a persistent launch over n work items (one per thread and step of the sweep): blocks
+// of 512 threads, as few as the items fill, since a reduction waits for every block (1.5 us on
+// 8 blocks, 2.4 on 148); past one block per SM the blocks grow to what the kernel's registers
+// allow and the sweep takes several steps.
+template <auto Kernel>
+static int launch_coop(long long n, void** params, cudaStream_t st) {
+    static const int maxThreads = [] {
+        cudaFuncAttributes f;
+        return cudaFuncGetAttributes(&f, (const void*)Kernel) == cudaSuccess ? std::min(f.maxThreadsPerBlock, GR_THREADS) : 256;
+    }();
+    const int nsm = sm_count();
+    int block = 128;
+    while (block < maxThreads && n > (long long)block * std::min(nsm, 32)) block = std::min(2 * block, maxThreads);
+    const int grid = (int)std::min<long long>(nsm, (n + block - 1) / block);
+    CB_CUDA(cudaLaunchCooperativeKernel((const void*)Kernel, dim3(grid), dim3(block), params, 0, st));
+    return 0;
+}
+template <auto Kernel, class Op>
+static int launch_coop(const Op& op, KArgs& args, cudaStream_t st) {
+    void* params[2] = {const_cast<Op*>(&op), &args};
+    return launch_coop<Kernel>(args.N, params, st);
 }
 
-template <class K>
-static int launch_coop(K kernel, int grid, KArgs& args, const void* op, cudaStream_t st) {
-    void* params[2] = {const_cast<void*>(op), &args};
-    CB_CUDA(cudaLaunchCooperativeKernel((const void*)kernel, dim3(grid), dim3(KB), params, 0, st));
+size_t krylov_partial_doubles() { return gr_doubles(sm_count()); }
+
+template <class Op>
+static int prepare(const Op& A, const Lat& L, const KspWork& w, cudaStream_t st) {
+    inv_diag_kernel<Op><<<grid_for(L.N, 256), 256, 0, st>>>(A, L.N, w.invD, w.partials);
+    CB_CHECK_LAUNCH();
     return 0;
 }
 
 static KArgs make_args(const Lat& L, const KspWork& w, const double* b, double* x, double rtol, int maxit, double atol) {
     KArgs a;
-    a.b = b; a.x = x; a.r = w.r; a.rp = w.rp;
+    a.b = b; a.x = x; a.r = w.r; a.rp = w.rp; a.s = w.r + L.PS;
     a.p[0] = w.p[0]; a.p[1] = w.p[1]; a.v[0] = w.v[0]; a.v[1] = w.v[1];
     a.t = w.t; a.invD = w.invD; a.partials = w.partials; a.out = w.out;
     a.N = L.N; a.PS = L.PS; a.rtol = rtol; a.atol = atol; a.maxit = maxit;
     a.project = 0;
     a.skip_if_ok = nullptr;
     a.fallbacks = nullptr;
+    for (int q = 0; q < 3; ++q) a.cs[q] = w.cs[q];
     return a;
+}
+
+// The two CG launches: the scaled form, and the general one for the systems it does not take
+// (each returns at once where the other runs).  Groups of two cells where the rows are even.
+template <class Op>
+static int run_cg(const Op& A, const Lat& L, const KspWork& w, KArgs& a, cudaStream_t st) {
+    if (w.cs[0] && L.N < (1ll << 31) - 2 * L.nIJ) {
+        CB_CUDA(cudaMemsetAsync(&w.out->general, 0, sizeof(int), st));
+        scale_kernel<Op, double><<<grid_for(L.N, 256), 256, 0, st>>>(A, L.N, w.invD, w.cs[0], w.cs[1], w.cs[2], &w.out->general, w.partials);
+        CB_CHECK_LAUNCH();
+        auto al = [](const void* p) { return ((uintptr_t)p & 15u) == 0; };
+        const bool v2 = L.nI % 2 == 0 && al(a.r) && al(a.v[0]) && al(a.p[0]) && al(a.x) &&
+                        al(a.cs[0]) && al(a.cs[1]) && al(a.cs[2]) && al(diag_plane(A));
+        void* params[2] = {const_cast<Op*>(&A), &a};
+        if (v2 ? launch_coop<cgs_kernel<Op, 2>>(L.N / 2, params, st) : launch_coop<cgs_kernel<Op, 1>>(L.N, params, st)) return 1;
+    } else
+        for (int q = 0; q < 3; ++q) a.cs[q] = nullptr;
+    if (prepare(A, L, w, st)) return 1;
+    return launch_coop<cg1_kernel<Op>>(A, a, st);
+}
+
+// Groups of two cells where the rows are even.
+static int run_bicgstab(const OpSym& A, const Lat& L, KArgs& a, cudaStream_t st) {
+    auto al = [](const void* p) { return ((uintptr_t)p & 15u) == 0; };
+    const bool v2 = L.nI % 2 == 0 && al(a.r) && al(a.s) && al(a.rp) && al(a.p[0]) && al(a.p[1]) && al(a.v[0]) && al(a.v[1]) && al(a.t) &&
+                    al(a.invD) && al(a.x) && al(A.aP) && al(A.aE) && al(A.aN) && al(A.aT);
+    void* params[2] = {const_cast<OpSym*>(&A), &a};
+    return v2 ? launch_coop<bicgstab_kernel<1, OpSym, 2>>(L.N / 2, params, st) : launch_coop<bicgstab_kernel<1, OpSym, 1>>(L.N, params, st);
 }
 
 int ksp_bicgstab(const Op7& A, int nr, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit,
                  cudaStream_t st, double atol) {
-    inv_diag_kernel<Op7><<<grid_for(L.N, 256), 256, 0, st>>>(A, L.N, w.invD);
-    CB_CHECK_LAUNCH();
+    if (prepare(A, L, w, st)) return 1;
     KArgs a = make_args(L, w, b, x, rtol, maxit, atol);
     if (nr == 3) {
-        static int G = 0;
-        if (!G) G = coop_grid(bicgstab_kernel<3, Op7>);
-        return launch_coop(bicgstab_kernel<3, Op7>, G, a, &A, st);
+        void* params[2] = {const_cast<Op7*>(&A), &a};
+        CB_CUDA(cudaLaunchCooperativeKernel((const void*)bicgstab3_kernel<3, Op7>, dim3(2 * sm_count()), dim3(KB), params, 0, st));
+        return 0;
     }
-    static int G1 = 0;
-    if (!G1) G1 = coop_grid(bicgstab_kernel<1, Op7>);
-    return launch_coop(bicgstab_kernel<1, Op7>, G1, a, &A, st);
+    return launch_coop<bicgstab_kernel<1, Op7, 1>>(A, a, st);
 }
 
 int ksp_bicgstab_sym(const OpSym& A, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit,
                      cudaStream_t st, int project, double atol) {
-    inv_diag_kernel<OpSym><<<grid_for(L.N, 256), 256, 0, st>>>(A, L.N, w.invD);
-    CB_CHECK_LAUNCH();
+    if (prepare(A, L, w, st)) return 1;
     KArgs a = make_args(L, w, b, x, rtol, maxit, atol);
     a.project = project;
-    static int G = 0;
-    if (!G) G = coop_grid(bicgstab_kernel<1, OpSym>);
-    return launch_coop(bicgstab_kernel<1, OpSym>, G, a, &A, st);
+    return run_bicgstab(A, L, a, st);
 }
 
 int ksp_cg(const OpSym& A, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit, cudaStream_t st,
            int project, double atol) {
-    inv_diag_kernel<OpSym><<<grid_for(L.N, 256), 256, 0, st>>>(A, L.N, w.invD);
-    CB_CHECK_LAUNCH();
     KArgs a = make_args(L, w, b, x, rtol, maxit, atol);
     a.project = project;
-    static int G = 0;
-    if (!G) G = coop_grid(cg1_kernel<OpSym>);
-    return launch_coop(cg1_kernel<OpSym>, G, a, &A, st);
+    return run_cg(A, L, w, a, st);
 }
 
 int ksp_cg7(const Op7& A, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit, cudaStream_t st,
             double atol) {
-    inv_diag_kernel<Op7><<<grid_for(L.N, 256), 256, 0, st>>>(A, L.N, w.invD);
-    CB_CHECK_LAUNCH();
     KArgs a = make_args(L, w, b, x, rtol, maxit, atol);
-    static int G = 0;
-    if (!G) G = coop_grid(cg1_kernel<Op7>);
-    return launch_coop(cg1_kernel<Op7>, G, a, &A, st);
+    return run_cg(A, L, w, a, st);
 }
 
 int ksp_csr(const OpCSR& A, int method, long long n, const double* b, double* x, const KspWork& w, double rtol, int maxit,
             cudaStream_t st, double atol) {
-    inv_diag_kernel<OpCSR><<<grid_for(n, 256), 256, 0, st>>>(A, n, w.invD);
-    CB_CHECK_LAUNCH();
     Lat L;
     std::memset(&L, 0, sizeof(L));
     L.nI = (int)n; L.nJ = 1; L.nK = 1; L.N = n; L.nIJ = n; L.H = 0; L.PS = n;   // unpadded vectors
+    if (prepare(A, L, w, st)) return 1;
     KArgs a = make_args(L, w, b, x, rtol, maxit, atol);
-    if (method == CAFFE_KSP_CG_JACOBI_INT) {
-        static int G = 0;
-        if (!G) G = coop_grid(cg1_kernel<OpCSR>);
-        return launch_coop(cg1_kernel<OpCSR>, G, a, &A, st);
-    }
-    static int G = 0;
-    if (!G) G = coop_grid(bicgstab_kernel<1, OpCSR>);
-    return launch_coop(bicgstab_kernel<1, OpCSR>, G, a, &A, st);
+    for (int q = 0; q < 3; ++q) a.cs[q] = nullptr;
+    return method == CAFFE_KSP_CG_JACOBI_INT ? launch_coop<cg1_kernel<OpCSR>>(A, a, st) : launch_coop<bicgstab_kernel<1, OpCSR, 1>>(A, a, st);
 }
 
-int krylov_grid_size(int which) {
-    switch (which) {
-        case 0: return coop_grid(bicgstab_kernel<3, Op7>);
-        case 1: return coop_grid(bicgstab_kernel<1, OpSym>);
-        case 2: return coop_grid(cg1_kernel<OpSym>);
-        case 4: return coop_grid(cg1_kernel<Op7>);
-        case 5: return coop_grid(bicgstab_kernel<1, OpCSR>);
-        case 6: return coop_grid(cg1_kernel<OpCSR>);
-        default: return coop_grid(bicgstab_kernel<1, Op7>);
-    }
-}
-
-
-int ksp_mixed_sym(const OpSym& A, int method, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit,
-                  double inner_rtol, cudaStream_t st, int project, double atol) {
-    cast_sym_kernel<<<grid_for(L.N, 256), 256, 0, st>>>(A, L.N, w.fA[0], w.fA[1], w.fA[2], w.fA[3], w.finvD);
-    CB_CHECK_LAUNCH();
-    OpSymF Af;
-    Af.aP = w.fA[0]; Af.aE = w.fA[1]; Af.aN = w.fA[2]; Af.aT = w.fA[3];
-    Af.nI = A.nI; Af.nIJ = A.nIJ; Af.gh = A.gh;
+int ksp_mixed_sym(const OpSym& A, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit,
+                  cudaStream_t st, int project, double atol) {
     MxArgs m;
     m.b = b; m.x = x;
-    m.r[0] = w.fr[0]; m.r[1] = w.fr[1]; m.w[0] = w.fw[0]; m.w[1] = w.fw[1]; m.s[0] = w.fs[0]; m.s[1] = w.fs[1];
-    m.p = w.fp; m.e = w.fe; m.v[0] = w.fv[0]; m.v[1] = w.fv[1]; m.t = w.ft; m.invD = w.finvD;
-    m.partials = w.partials; m.out = w.out; m.N = L.N; m.rtol = rtol; m.atol = atol; m.maxit = maxit; m.eta = inner_rtol;
-    m.project = project; m.inner_max = 100000;
-    void* params[3] = {const_cast<OpSym*>(&A), &Af, &m};
-    if (method == CAFFE_KSP_CG_JACOBI_INT) {
-        static int G = 0;
-        if (!G) { int nb = 0; cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, mixed_kernel<OpSym, 0>, KB, 0); G = (nb < 1 ? 1 : (nb > 4 ? 4 : nb)) * sm_count(); }
-        CB_CUDA(cudaLaunchCooperativeKernel((const void*)mixed_kernel<OpSym, 0>, dim3(G), dim3(KB), params, 0, st));
-    } else {
-        static int G = 0;
-        if (!G) { int nb = 0; cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, mixed_kernel<OpSym, 1>, KB, 0); G = (nb < 1 ? 1 : (nb > 4 ? 4 : nb)) * sm_count(); }
-        CB_CUDA(cudaLaunchCooperativeKernel((const void*)mixed_kernel<OpSym, 1>, dim3(G), dim3(KB), params, 0, st));
-    }
-    return 0;
+    m.r = w.fr; m.q = w.fq; m.p = w.fp; m.e = w.fe; m.d = w.fd; m.S = w.invD;
+    for (int q = 0; q < 3; ++q) m.cs[q] = w.fB[q];
+    m.partials = w.partials; m.out = w.out; m.N = L.N; m.rtol = rtol; m.atol = atol; m.maxit = maxit; m.project = project;
+    CB_CUDA(cudaMemsetAsync(&w.out->general, 0, sizeof(int), st));
+    cast_kernel<<<grid_for(L.N, 256), 256, 0, st>>>(L.N, A.aP, w.fd);
+    scale_kernel<OpSym, float><<<grid_for(L.N, 256), 256, 0, st>>>(A, L.N, w.invD, w.fB[0], w.fB[1], w.fB[2], &w.out->general, w.partials);
+    CB_CHECK_LAUNCH();
+    void* params[2] = {const_cast<OpSym*>(&A), &m};
+    // cell arrays start 16-byte aligned; groups of 16 bytes where the rows are multiples of them
+    return L.nI % 4 == 0 ? launch_coop<mixed_cg_kernel<4>>(L.N / 4, params, st) : launch_coop<mixed_cg_kernel<1>>(L.N, params, st);
 }
 
 int ksp_fallback_sym(const OpSym& A, int method, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit,
                      cudaStream_t st, int project, const int* status, int* fallbacks, double atol) {
     // plain FP64 re-solve from zero, executed only when *status (the previous solve's) is non-zero
-    inv_diag_kernel<OpSym><<<grid_for(L.N, 256), 256, 0, st>>>(A, L.N, w.invD);
-    CB_CHECK_LAUNCH();
     KArgs a = make_args(L, w, b, x, rtol, maxit, atol);
     a.project = project;
     a.skip_if_ok = status;
     a.fallbacks = fallbacks;
-    if (method == CAFFE_KSP_CG_JACOBI_INT) {
-        static int G = 0;
-        if (!G) G = coop_grid(cg1_kernel<OpSym>);
-        return launch_coop(cg1_kernel<OpSym>, G, a, &A, st);
-    }
-    static int G = 0;
-    if (!G) G = coop_grid(bicgstab_kernel<1, OpSym>);
-    return launch_coop(bicgstab_kernel<1, OpSym>, G, a, &A, st);
+    if (method == CAFFE_KSP_CG_JACOBI_INT) return run_cg(A, L, w, a, st);
+    if (prepare(A, L, w, st)) return 1;
+    return run_bicgstab(A, L, a, st);
 }
 
 }  // namespace cb

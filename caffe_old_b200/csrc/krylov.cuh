@@ -6,13 +6,14 @@ namespace cb {
 
 // Immersed-boundary ghost rows in ELL-9 form, sorted by cell (IbPiso.cpp:119-190):
 // col[9g + 0] is the ghost cell itself, col[9g + 1..8] the interpolation stencil (-1 for a
-// dropped column), val[9g + m] the coefficients; bits marks ghost cells (one bit per cell).
+// dropped column), val[9g + m] the coefficients; words has one
+// entry per 32 cells: a bit per ghost cell, and the number of ghost cells before them.
 struct GhostRows {
     int n;
     const int* cell;
     const int* col;
     const double* val;
-    const uint32_t* bits;
+    const uint2* words;
 };
 
 // Non-symmetric 7-point operator: 7 per-cell coefficient arrays (momentum, Simple.cpp:162-171).
@@ -49,11 +50,12 @@ struct KspOut {
     double relres[3];
     int status[3];      // 0 converged, 1 maxit, 2 breakdown, 3 non-finite
     int cascades;       // learned solve only: 1 when its network stage handed over to the pyramid stage
+    int general;        // CG: set when the scaled form does not apply to the system
     int net_iters;      // learned solve only: inner iterations run with the network in the preconditioner
 };
 
 // Workspace for up to NR = 3 right-hand sides; every array is a halo-padded cell array of
-// 3 planes (the single right-hand-side CG also uses plane 1 of r as a second buffer).
+// 3 planes (a single right-hand side also uses the plane after r as a second buffer).
 struct KspWork {
     double* r;
     double* rp;
@@ -61,18 +63,13 @@ struct KspWork {
     double* v[2];
     double* t;
     double* invD;     // one plane
-    double* partials; // grid x 8 doubles
+    double* cs[3];    // CG: off-diagonal planes of the scaled operator (null: the unscaled form runs)
+    double* partials; // slots of the grid reductions: krylov_partial_doubles()
     KspOut* out;      // device
     // single-precision workspace of the mixed-precision solver (halo-padded float cell arrays)
-    float* fr[2];
-    float* fw[2];
-    float* fs[2];
-    float* fp;
-    float* fe;
-    float* finvD;
-    float* fA[4];     // aP aE aN aT in FP32
-    float* fv[2];     // extra vectors of the FP32 BiCGStab inner solver
-    float* ft;
+    float *fr, *fq, *fp, *fe;
+    float* fd;        // diagonal
+    float* fB[3];     // off-diagonal planes of the scaled operator
 };
 
 // Every solve stops once ||b - A x|| <= max(rtol ||b||, atol) in the FP64 true residual (the
@@ -86,12 +83,10 @@ int ksp_cg(const OpSym& A, const double* b, double* x, const Lat& L, const KspWo
            int project = 0, double atol = 0.);
 int ksp_cg7(const Op7& A, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit, cudaStream_t st,
             double atol = 0.);
-// FP64 iterative refinement around FP32 inner solves on the symmetric p' operator: CG inner
-// (method CAFFE_KSP_CG_JACOBI, symmetric systems) or BiCGStab inner (ghost rows).
-// inner_rtol: relative reduction each inner solve aims for.  out->iters counts inner
-// iterations; the outer count goes to *outer_iters (device int, may be null).
-int ksp_mixed_sym(const OpSym& A, int method, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit,
-                  double inner_rtol, cudaStream_t st, int project, double atol = 0.);
+// FP64 iterative refinement around FP32 CG on the symmetric p' operator (no ghost rows).
+// out->iters[0] counts the FP32 iterations, iters[1] the refinements.
+int ksp_mixed_sym(const OpSym& A, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit,
+                  cudaStream_t st, int project, double atol = 0.);
 // Plain FP64 re-solve that runs only when *status is non-zero (the fallback of a mixed or
 // learned solve), decided on the device without a host round trip.
 int ksp_fallback_sym(const OpSym& A, int method, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit,
@@ -100,9 +95,7 @@ int ksp_fallback_sym(const OpSym& A, int method, const double* b, double* x, con
 // with Jacobi preconditioning, the same persistent kernels as the lattice solves.
 int ksp_csr(const OpCSR& A, int method, long long n, const double* b, double* x, const KspWork& w, double rtol, int maxit,
             cudaStream_t st, double atol = 0.);
-// Blocks of the cooperative grid a solve launches: 0 BiCGStab on 3 right-hand sides (Op7),
-// 1 BiCGStab (OpSym), 2 CG (OpSym), 3 BiCGStab (Op7), 4 CG (Op7), 5 BiCGStab (OpCSR), 6 CG (OpCSR).  The block partials of a
-// solve take 2 x grid x 8 doubles.
-int krylov_grid_size(int which);
+// Doubles of slot memory (KspWork::partials) that the reductions of a solve take on this device.
+size_t krylov_partial_doubles();
 
 }  // namespace cb

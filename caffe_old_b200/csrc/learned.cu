@@ -64,6 +64,7 @@
 #include "cnn.cuh"
 #include "krylov.cuh"
 #include "learned.cuh"
+#include "stencil.cuh"
 
 namespace cb {
 
@@ -186,11 +187,11 @@ __global__ void __launch_bounds__(LB) outer_residual_kernel(OpSym A, long long N
                    + __ldg(A.aN + c) * x[c + A.nI] + __ldg(A.aN + c - A.nI) * x[c - A.nI]
                    + __ldg(A.aT + c) * x[c + A.nIJ] + __ldg(A.aT + c - A.nIJ) * x[c - A.nIJ];
         if (A.gh.n > 0) {
-            uint32_t w = __ldg(A.gh.bits + (c >> 5));
-            if ((w >> (c & 31)) & 1u) {
-                int lo = 0, hi = A.gh.n;
-                while (lo < hi) { int mid = (lo + hi) >> 1; if (__ldg(A.gh.cell + mid) < c) lo = mid + 1; else hi = mid; }
+            const uint2 w = __ldg(A.gh.words + (c >> 5));
+            if (is_ghost(w, c)) {
+                const int lo = ghost_index(w, c);
                 double s = 0.;
+#pragma unroll 1
                 for (int m = 0; m < 9; ++m) { int col = __ldg(A.gh.col + 9 * lo + m); if (col >= 0) s += __ldg(A.gh.val + 9 * lo + m) * x[col]; }
                 y = s;
             }
@@ -938,11 +939,11 @@ __device__ __forceinline__ float applyF(const OpSymF32& A, long long c, X&& x) {
     float y = __ldg(A.aP + c) * x(c) + __ldg(A.aE + c) * x(c + 1) + __ldg(A.aE + c - 1) * x(c - 1) + __ldg(A.aN + c) * x(c + A.nI)
               + __ldg(A.aN + c - A.nI) * x(c - A.nI) + __ldg(A.aT + c) * x(c + A.nIJ) + __ldg(A.aT + c - A.nIJ) * x(c - A.nIJ);
     if (A.gh.n > 0) {
-        uint32_t w = __ldg(A.gh.bits + (c >> 5));
-        if ((w >> (c & 31)) & 1u) {
-            int lo = 0, hi = A.gh.n;
-            while (lo < hi) { int mid = (lo + hi) >> 1; if (__ldg(A.gh.cell + mid) < c) lo = mid + 1; else hi = mid; }
+        const uint2 w = __ldg(A.gh.words + (c >> 5));
+        if (is_ghost(w, c)) {
+            const int lo = ghost_index(w, c);
             float s = 0.f;
+#pragma unroll 1
             for (int m = 0; m < 9; ++m) { int col = __ldg(A.gh.col + 9 * lo + m); if (col >= 0) s += (float)__ldg(A.gh.val + 9 * lo + m) * x(col); }
             y = s;
         }
@@ -1182,7 +1183,7 @@ __device__ __forceinline__ void spmv4(const OpSymF32& A, const float* x, long lo
     for (int m = 0; m < 4; ++m)
         Y[m] = P[m] * X[m] + E[m] * xr[m] + W[m] * xl[m] + Nn[m] * XN[m] + Sn[m] * XS[m] + T[m] * XT[m] + B[m] * XB[m];
     if (A.gh.n > 0) {
-        const uint32_t bits = (__ldg(A.gh.bits + (c >> 5)) >> (c & 31)) & 0xFu;
+        const uint32_t bits = (__ldg(A.gh.words + (c >> 5)).x >> (c & 31)) & 0xFu;
         if (bits)
 #pragma unroll
             for (int m = 0; m < 4; ++m)
@@ -1967,11 +1968,11 @@ __global__ void __launch_bounds__(LB) snapshot_pair_kernel(OpSym A, long long N,
                    + __ldg(A.aN + c) * xk[c + A.nI] + __ldg(A.aN + c - A.nI) * xk[c - A.nI]
                    + __ldg(A.aT + c) * xk[c + A.nIJ] + __ldg(A.aT + c - A.nIJ) * xk[c - A.nIJ];
         if (A.gh.n > 0) {
-            uint32_t w = __ldg(A.gh.bits + (c >> 5));
-            if ((w >> (c & 31)) & 1u) {
-                int lo = 0, hi = A.gh.n;
-                while (lo < hi) { int mid = (lo + hi) >> 1; if (__ldg(A.gh.cell + mid) < c) lo = mid + 1; else hi = mid; }
+            const uint2 w = __ldg(A.gh.words + (c >> 5));
+            if (is_ghost(w, c)) {
+                const int lo = ghost_index(w, c);
                 double s = 0.;
+#pragma unroll 1
                 for (int m = 0; m < 9; ++m) { int col = __ldg(A.gh.col + 9 * lo + m); if (col >= 0) s += __ldg(A.gh.val + 9 * lo + m) * xk[col]; }
                 y = s;
             }

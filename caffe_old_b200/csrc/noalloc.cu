@@ -33,8 +33,8 @@ namespace cb {
 namespace {
 
 constexpr size_t SCRATCH_BYTES = size_t(16) << 20;
-// 2 buffers x 8 doubles x up to 1024 blocks of partials: the cooperative grid is capped at 4
-// blocks per SM, so this covers GPUs of up to 256 SMs (B200: 148); checked per call
+// slots of the grid reductions: 128 bytes per SM, far below this;
+// checked per call
 constexpr size_t PARTIAL_BYTES = size_t(128) << 10;
 constexpr int MAX_DEVICES = 64;
 
@@ -91,12 +91,9 @@ extern "C" int caffe_ksp7_solve_device_noalloc(int nI, int nJ, int nK, const dou
                   std::to_string(SCRATCH_BYTES) + " the no-allocation solver holds; use caffe_ksp7_solve_device");
         return 1;
     }
-    // the block partials of the cooperative solve (2 buffers x grid x 8 doubles) must fit their
-    // fixed slice: the grid is at most 4 blocks per SM
-    const int grid = krylov_grid_size(method == CAFFE_KSP_CG_JACOBI ? 4 : 3);
-    if ((size_t)2 * grid * 8 * sizeof(double) > PARTIAL_BYTES) {
-        set_error("caffe_ksp7_solve_device_noalloc: the solver's grid of " + std::to_string(grid) +
-                  " blocks needs more block-partial space than the no-allocation workspace holds");
+    // the reduction slots of the solve must fit their fixed slice
+    if (krylov_partial_doubles() * sizeof(double) > PARTIAL_BYTES) {
+        set_error("caffe_ksp7_solve_device_noalloc: the solver's reductions need more space than the no-allocation workspace holds");
         return 1;
     }
     void* base = nullptr;
@@ -122,7 +119,7 @@ extern "C" int caffe_ksp7_solve_device_noalloc(int nI, int nJ, int nK, const dou
     Op7 A;
     for (int q = 0; q < 7; ++q) A.a[q] = d_coef7 + (size_t)q * L.N;   // coefficients are read at their own row only
     A.nI = L.nI; A.nIJ = L.nIJ;
-    A.gh.n = 0; A.gh.cell = nullptr; A.gh.col = nullptr; A.gh.val = nullptr; A.gh.bits = nullptr;
+    A.gh.n = 0; A.gh.cell = nullptr; A.gh.col = nullptr; A.gh.val = nullptr; A.gh.words = nullptr;
     int rc = method == CAFFE_KSP_CG_JACOBI ? ksp_cg7(A, b, x, L, w, rtol, maxit, st) : ksp_bicgstab(A, 1, b, x, L, w, rtol, maxit, st);
     if (rc) return rc;
     KspOut o;

@@ -1,0 +1,74 @@
+"""The persistent Krylov kernels at the edges of their launch shapes and dispatch: one cell, rows too
+short or odd for the two-cell groups, one plane, sweeps of several steps, diagonals of either
+sign, and the systems the scaled CG hands to the general one (mixed signs of the diagonal, a
+matrix that is not symmetric).
+
+Tolerance: the solve stops at a true relative residual of 1e-12, so the residual of the returned x,
+evaluated on the host, is within 1e-11; on small systems x agrees with a dense solve to 1e-9 (condition
+numbers up to about 1e3)."""
+import numpy as np
+import pytest
+
+from caffe_old_b200 import _lib
+
+from test_zz_no_alloc import seven_point_residual, seven_point_system
+
+pytestmark = pytest.mark.gpu
+
+RTOL = 1e-12
+
+
+def dense(shape, coef):
+    nI, nJ, _ = shape
+    N = coef.shape[1]
+    A = np.diag(coef[0])
+    for q, off in ((1, 1), (3, nI), (5, nI * nJ)):
+        for c in range(N - off):
+            A[c, c + off] += coef[q][c]
+            A[c + off, c] += coef[q + 1][c + off]
+    return A
+
+
+@pytest.mark.parametrize("sign", [-1.0, 1.0])
+@pytest.mark.parametrize("method", ["cg_jacobi", "bicgstab_jacobi"])
+@pytest.mark.parametrize("shape", [(1, 1, 1), (2, 1, 1), (3, 1, 1), (1, 7, 2), (2, 2, 2), (33, 4, 3), (64, 3, 2), (129, 64, 33), (200, 120, 31)])
+def test_solution_at_the_edges_of_the_launch_shapes(shape, method, sign):
+    N = int(np.prod(shape))
+    if N > 8:
+        coef, b = seven_point_system(shape, 11, True)
+    else:   # the generator wants a neighbour in every direction
+        coef, b = np.zeros((7, N)), np.arange(1.0, N + 1.0)
+        i, j, k = np.arange(N) % shape[0], (np.arange(N) // shape[0]) % shape[1], np.arange(N) // (shape[0] * shape[1])
+        for q, inside in enumerate((i < shape[0] - 1, i > 0, j < shape[1] - 1, j > 0, k < shape[2] - 1, k > 0)):
+            coef[q + 1][inside] = 1.0 + 0.1 * (q // 2)
+        coef[0] = -coef[1:].sum(axis=0) - 0.15
+    coef = sign * coef
+    x, _, rr, st = _lib.ksp7_solve(shape, coef, b, method, RTOL, 20000)
+    assert st == 0 and rr <= RTOL
+    if N <= 500:
+        ref = np.linalg.solve(dense(shape, coef), b)
+        assert np.linalg.norm(x - ref) <= 1e-9 * np.linalg.norm(ref)
+    else:
+        assert seven_point_residual(shape, coef, x, b) <= 1e-11
+
+
+def test_cg_on_a_diagonal_of_mixed_signs():
+    shape = (6, 5, 4)
+    rng = np.random.default_rng(3)
+    coef = np.zeros((7, 120))
+    coef[0] = rng.uniform(1.0, 2.0, 120) * np.where(np.arange(120) % 3 == 0, -1.0, 1.0)
+    b = rng.standard_normal(120)
+    x, _, _, st = _lib.ksp7_solve(shape, coef, b, "cg_jacobi", RTOL, 100)
+    assert st == 0
+    assert np.linalg.norm(x - b / coef[0]) <= 1e-11 * np.linalg.norm(x)
+
+
+def test_cg_on_a_matrix_that_is_not_symmetric_runs_the_general_form():
+    """Nearly symmetric: CG still converges, and only the operator as given leaves a small residual."""
+    shape = (12, 9, 5)
+    coef, b = seven_point_system(shape, 4, True)
+    coef = coef.copy()
+    coef[2] *= 1.0 + 1e-9
+    x, _, rr, st = _lib.ksp7_solve(shape, coef, b, "cg_jacobi", RTOL, 5000)
+    assert st == 0 and rr <= RTOL
+    assert seven_point_residual(shape, coef, x, b) <= 1e-11
