@@ -415,10 +415,11 @@ int ph_solve_pcorr(caffe_dev* h) {
                            project, h->netMode, h->kw.out, h->st, h->cs.p_atol);
         if (!rc) rc = ksp_fallback_sym(A, method, h->pb, h->pc, h->L, h->kw, h->cs.p_rtol, h->cs.maxit, h->st, 0,
                                        &h->kw.out->status[0], &h->acc->fallbacks, h->cs.p_atol);
-    } else if (h->cs.p_form == CAFFE_P_MIXED && sym) {
+    } else if (h->cs.p_form == CAFFE_P_MIXED && sym && !ksp_small_fits(h->L)) {
         // FP32 CG inside FP64 refinement (whichever method the case names: the system is symmetric);
         // the plain FP64 solve re-runs on the device when the refinement does not reach the
-        // tolerance.  Systems with ghost rows take the FP64 BiCGStab below (krylov.cu)
+        // tolerance.  Systems with ghost rows take the FP64 BiCGStab below (krylov.cu), and those that one
+        // cluster holds the FP64 solve there, where an iteration moves nothing and FP32 saves nothing
         rc = ksp_mixed_sym(A, h->pb, h->pc, h->L, h->kw, h->cs.p_rtol, h->cs.maxit, h->st, project, h->cs.p_atol);
         if (!rc) rc = ksp_fallback_sym(A, method, h->pb, h->pc, h->L, h->kw, h->cs.p_rtol, h->cs.maxit, h->st, 0,
                                        &h->kw.out->status[0], &h->acc->fallbacks, h->cs.p_atol);

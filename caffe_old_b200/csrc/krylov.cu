@@ -1100,6 +1100,7 @@ static int run_bicgstab(const OpSym& A, const Lat& L, KArgs& a, cudaStream_t st)
 
 int ksp_bicgstab(const Op7& A, int nr, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit,
                  cudaStream_t st, double atol) {
+    if (ksp_small_fits(L)) return ksp_small(A, false, nr, b, x, L, w, rtol, maxit, st, 0, atol);
     if (prepare(A, L, w, st)) return 1;
     KArgs a = make_args(L, w, b, x, rtol, maxit, atol);
     if (nr == 3) {
@@ -1112,6 +1113,7 @@ int ksp_bicgstab(const Op7& A, int nr, const double* b, double* x, const Lat& L,
 
 int ksp_bicgstab_sym(const OpSym& A, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit,
                      cudaStream_t st, int project, double atol) {
+    if (ksp_small_fits(L)) return ksp_small(A, false, b, x, L, w, rtol, maxit, st, project, atol, nullptr, nullptr);
     if (prepare(A, L, w, st)) return 1;
     KArgs a = make_args(L, w, b, x, rtol, maxit, atol);
     a.project = project;
@@ -1120,6 +1122,7 @@ int ksp_bicgstab_sym(const OpSym& A, const double* b, double* x, const Lat& L, c
 
 int ksp_cg(const OpSym& A, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit, cudaStream_t st,
            int project, double atol) {
+    if (ksp_small_fits(L)) return ksp_small(A, true, b, x, L, w, rtol, maxit, st, project, atol, nullptr, nullptr);
     KArgs a = make_args(L, w, b, x, rtol, maxit, atol);
     a.project = project;
     return run_cg(A, L, w, a, st);
@@ -1127,6 +1130,7 @@ int ksp_cg(const OpSym& A, const double* b, double* x, const Lat& L, const KspWo
 
 int ksp_cg7(const Op7& A, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit, cudaStream_t st,
             double atol) {
+    if (ksp_small_fits(L)) return ksp_small(A, true, 1, b, x, L, w, rtol, maxit, st, 0, atol);
     KArgs a = make_args(L, w, b, x, rtol, maxit, atol);
     return run_cg(A, L, w, a, st);
 }
@@ -1136,6 +1140,7 @@ int ksp_csr(const OpCSR& A, int method, long long n, const double* b, double* x,
     Lat L;
     std::memset(&L, 0, sizeof(L));
     L.nI = (int)n; L.nJ = 1; L.nK = 1; L.N = n; L.nIJ = n; L.H = 0; L.PS = n;   // unpadded vectors
+    if (ksp_small_fits(L)) return ksp_small(A, method == CAFFE_KSP_CG_JACOBI_INT, b, x, L, w, rtol, maxit, st, atol);
     if (prepare(A, L, w, st)) return 1;
     KArgs a = make_args(L, w, b, x, rtol, maxit, atol);
     for (int q = 0; q < 3; ++q) a.cs[q] = nullptr;
@@ -1161,6 +1166,8 @@ int ksp_mixed_sym(const OpSym& A, const double* b, double* x, const Lat& L, cons
 int ksp_fallback_sym(const OpSym& A, int method, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit,
                      cudaStream_t st, int project, const int* status, int* fallbacks, double atol) {
     // plain FP64 re-solve from zero, executed only when *status (the previous solve's) is non-zero
+    if (ksp_small_fits(L))
+        return ksp_small(A, method == CAFFE_KSP_CG_JACOBI_INT, b, x, L, w, rtol, maxit, st, project, atol, status, fallbacks);
     KArgs a = make_args(L, w, b, x, rtol, maxit, atol);
     a.project = project;
     a.skip_if_ok = status;

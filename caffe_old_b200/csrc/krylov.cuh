@@ -95,6 +95,15 @@ int ksp_fallback_sym(const OpSym& A, int method, const double* b, double* x, con
 // with Jacobi preconditioning, the same persistent kernels as the lattice solves.
 int ksp_csr(const OpCSR& A, int method, long long n, const double* b, double* x, const KspWork& w, double rtol, int maxit,
             cudaStream_t st, double atol = 0.);
+// The same solves inside one thread-block cluster, for systems whose vectors fit its registers and
+// shared memory (krylov_small.cu).  rhs right-hand sides PS apart, each solved by a cluster of its own.
+bool ksp_small_fits(const Lat& L);
+int ksp_small(const Op7& A, bool cgMethod, int rhs, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit,
+              cudaStream_t st, int project, double atol);
+int ksp_small(const OpSym& A, bool cgMethod, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit, cudaStream_t st,
+              int project, double atol, const int* skip_if_ok, int* fallbacks);
+int ksp_small(const OpCSR& A, bool cgMethod, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit, cudaStream_t st,
+              double atol);
 // Doubles of slot memory (KspWork::partials) that the reductions of a solve take on this device.
 size_t krylov_partial_doubles();
 

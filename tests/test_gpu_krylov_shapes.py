@@ -1,5 +1,6 @@
-"""The persistent Krylov kernels at the edges of their launch shapes and dispatch: one cell, rows too
-short or odd for the two-cell groups, one plane, sweeps of several steps, diagonals of either
+"""The persistent Krylov kernels at the edges of their launch shapes and dispatch: one cell, the sizes
+at which a cluster's blocks take more cells per thread or the system leaves the cluster (32768 cells, or
+planes too large for a halo), rows too short or odd for the two-cell groups, one plane, sweeps of several steps, diagonals of either
 sign, and the systems the scaled CG hands to the general one (mixed signs of the diagonal, a
 matrix that is not symmetric).
 
@@ -31,7 +32,8 @@ def dense(shape, coef):
 
 @pytest.mark.parametrize("sign", [-1.0, 1.0])
 @pytest.mark.parametrize("method", ["cg_jacobi", "bicgstab_jacobi"])
-@pytest.mark.parametrize("shape", [(1, 1, 1), (2, 1, 1), (3, 1, 1), (1, 7, 2), (2, 2, 2), (33, 4, 3), (64, 3, 2), (129, 64, 33), (200, 120, 31)])
+@pytest.mark.parametrize("shape", [(1, 1, 1), (2, 1, 1), (3, 1, 1), (1, 7, 2), (2, 2, 2), (33, 4, 3), (64, 3, 2), (64, 64, 1), (31, 13, 11), (25, 25, 25), (32, 32, 32), (33, 32, 32), (150, 150, 2),
+                                   (129, 64, 33), (200, 120, 31)])
 def test_solution_at_the_edges_of_the_launch_shapes(shape, method, sign):
     N = int(np.prod(shape))
     if N > 8:
