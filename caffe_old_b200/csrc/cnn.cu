@@ -385,7 +385,14 @@ size_t conv_smem_bytes() { return 1024 + W_BYTES + (size_t)NPL * 3 * BUF_BYTES; 
 // thread issues the chunk's four MMAs into four 128 x 16 FP32 accumulators in tensor memory that
 // stay there for all the CTA's chunks.  Two staging buffers alternate, so the next chunk is built
 // while the MMAs of the previous one run.  At the end every thread reads its accumulator row
-// (tcgen05.ld) and adds it to the FP32 gradient.
+// (tcgen05.ld) and stores it as the CTA's partial, and a second kernel adds the partials, in CTA order,
+// to the FP32 gradient.
+//
+// One launch serves every lattice of a layer (the levels of a pyramid, both signs of the odd form), as
+// the forward pass does: the chunks of all of them are dealt out to one set of CTAs, which flush once.
+// Adding each CTA's 6912 values to the gradient with atomics bounded a launch before, 83 us
+// whatever the level's size: the ten lattices of the 128x64x64 training case took 830 us a layer and
+// 89 us now, the sum of the partials included.
 namespace {
 constexpr int WG_CH = 16;                          // cells per chunk (the MMA's K)
 constexpr int WG_TILE_BYTES = 16 * 256;            // 16 row groups of 8 rows x 2 K groups x 16 bytes
@@ -393,20 +400,27 @@ constexpr int WG_A_BYTES = 4 * WG_TILE_BYTES;      // four M tiles
 constexpr int WG_B_BYTES = 512;                    // 16 x 16 bf16
 constexpr int WG_STAGE_BYTES = WG_A_BYTES + WG_B_BYTES;
 constexpr uint32_t WG_TMEM_COLS = 64;              // four 16-column accumulators
+constexpr int WG_W = 27 * 256;                     // values of a weight partial; 16 more of the bias, in FP64
 
 // byte offset of element (row m, K column k) in a canonical no-swizzle K-major tile
 __device__ __forceinline__ int kmajor_off(int m, int k) { return (m >> 3) * 256 + (k >> 3) * 128 + (m & 7) * 16 + (k & 7) * 2; }
 }  // namespace
 
-__global__ void __launch_bounds__(128) weight_grad_tc_kernel(Lat L, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dz,
-                                                             float* dW, float* db, int* err) {
+struct WgGroup {
+    Lat L[CONV_MAX_JOBS];
+    const __nv_bfloat16* x[CONV_MAX_JOBS];
+    const __nv_bfloat16* dz[CONV_MAX_JOBS];
+    long long end[CONV_MAX_JOBS];    // inclusive prefix sums of the jobs' chunk counts
+    int n;
+};
+
+__global__ void __launch_bounds__(128) weight_grad_tc_kernel(const __grid_constant__ WgGroup g, float* part, double* dbPart, int* err) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) uint64_t mbar[2];
     __shared__ uint32_t tmem_base_sh;
     const int warp = threadIdx.x >> 5;
-    const int chunksI = (L.nI + WG_CH - 1) / WG_CH;
-    const long long nChunks = (long long)chunksI * L.nJ * L.nK;
+    const long long nChunks = g.end[g.n - 1];
     if (threadIdx.x == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar[0])));
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar[1])));
@@ -425,11 +439,19 @@ __global__ void __launch_bounds__(128) weight_grad_tc_kernel(Lat L, const __nv_b
     uint32_t phase[2] = {0u, 0u};
     bool pending[2] = {false, false};
     bool failed = false;
-    float dbs[16];
+    // the bias gradient sums in FP64: the two evaluations of the odd form cancel in it (exactly so in the
+    // last layer), and the optimiser scales a gradient that should be zero up to a full step
+    double dbs[16];
 #pragma unroll
-    for (int o = 0; o < 16; ++o) dbs[o] = 0.f;
-    int n = 0;
-    for (long long u = blockIdx.x; u < nChunks; u += gridDim.x, ++n) {
+    for (int o = 0; o < 16; ++o) dbs[o] = 0.;
+    int n = 0, job = 0;
+    for (long long u0 = blockIdx.x; u0 < nChunks; u0 += gridDim.x, ++n) {
+        while (u0 >= g.end[job]) ++job;
+        const Lat& L = g.L[job];
+        const __nv_bfloat16* __restrict__ x = g.x[job];
+        const __nv_bfloat16* __restrict__ dz = g.dz[job];
+        const int chunksI = (L.nI + WG_CH - 1) / WG_CH;
+        const long long u = u0 - (job > 0 ? g.end[job - 1] : 0);
         const int s = n & 1;
         // the MMAs that read this staging buffer two chunks ago must have finished
         if (pending[s]) {
@@ -482,8 +504,8 @@ __global__ void __launch_bounds__(128) weight_grad_tc_kernel(Lat L, const __nv_b
             for (int o = 0; o < 8; ++o) {
                 *reinterpret_cast<__nv_bfloat16*>(B + kmajor_off(o, cell)) = vl[o];
                 *reinterpret_cast<__nv_bfloat16*>(B + kmajor_off(8 + o, cell)) = vh[o];
-                dbs[o] += __bfloat162float(vl[o]);
-                dbs[8 + o] += __bfloat162float(vh[o]);
+                dbs[o] += (double)__bfloat162float(vl[o]);
+                dbs[8 + o] += (double)__bfloat162float(vh[o]);
             }
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -514,6 +536,7 @@ __global__ void __launch_bounds__(128) weight_grad_tc_kernel(Lat L, const __nv_b
     } else if (n > 0) {
         asm volatile("tcgen05.fence::after_thread_sync;");
         // thread = accumulator row m = (tap, input channel) of each M tile
+        float* mine = part + (size_t)blockIdx.x * WG_W;
         const int m = threadIdx.x, tl = m >> 4, ch = m & 15;
 #pragma unroll 1
         for (int T = 0; T < 4; ++T) {
@@ -522,11 +545,17 @@ __global__ void __launch_bounds__(128) weight_grad_tc_kernel(Lat L, const __nv_b
             const int t = 8 * T + tl;
             if (t < 27)
 #pragma unroll
-                for (int o = 0; o < 16; ++o) atomicAdd(dW + (t * 16 + o) * 16 + ch, v[o]);
+                for (int o = 0; o < 16; ++o) mine[(t * 16 + o) * 16 + ch] = v[o];
         }
-        if (threadIdx.x < WG_CH)
+        if (warp == 0) {
+            // the chunk's cells are the lanes below WG_CH
 #pragma unroll
-            for (int o = 0; o < 16; ++o) atomicAdd(db + o, dbs[o]);
+            for (int o = 0; o < 16; ++o) {
+                double s = threadIdx.x < WG_CH ? dbs[o] : 0.;
+                for (int off = WG_CH / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+                if (threadIdx.x == 0) dbPart[(size_t)blockIdx.x * 16 + o] = s;
+            }
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
@@ -534,21 +563,71 @@ __global__ void __launch_bounds__(128) weight_grad_tc_kernel(Lat L, const __nv_b
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(WG_TMEM_COLS));
 }
 
-int launch_weight_grad(const Lat& L, const __nv_bfloat16* x, const __nv_bfloat16* dz, float* dW, float* db, int* err, cudaStream_t st) {
+// grad[p] += sum over the CTAs' partials, in CTA order per warp and then over the warps; the last block
+// sums the bias
+__global__ void __launch_bounds__(256) weight_grad_sum_kernel(const float* __restrict__ part, const double* __restrict__ dbPart, int ctas,
+                                                              float* grad, const int* err) {
+    __shared__ float sm[8][32];
+    __shared__ double sd[16][16];
+    if (*err) return;   // a CTA that failed left no partial
+    if (blockIdx.x == WG_W / 32) {
+        const int o = threadIdx.x & 15, w = threadIdx.x >> 4;
+        double s = 0.;
+        for (int c = w; c < ctas; c += 16) s += dbPart[(size_t)c * 16 + o];
+        sd[w][o] = s;
+        __syncthreads();
+        if (w == 0) {
+            for (int u = 1; u < 16; ++u) s += sd[u][o];
+            grad[WG_W + o] += (float)s;
+        }
+        return;
+    }
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, p = blockIdx.x * 32 + lane;
+    float s = 0.f;
+#pragma unroll 8
+    for (int c = w; c < ctas; c += 8) s += part[(size_t)c * WG_W + p];
+    sm[w][lane] = s;
+    __syncthreads();
+    if (w == 0) {
+        for (int u = 1; u < 8; ++u) s += sm[u][lane];
+        grad[p] += s;
+    }
+}
+
+static long long weight_grad_ctas() {
+    int dev = 0, nsm = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    return 4LL * nsm;
+}
+size_t weight_grad_part_floats() { return (size_t)weight_grad_ctas() * (WG_W + 32); }
+
+int launch_weight_grad_group(const WgSpec* specs, int n, float* grad, float* part, int* err, cudaStream_t st) {
     const size_t smem = 1024 + 2 * (size_t)WG_STAGE_BYTES;
     static bool attr = false;
     if (!attr) {
         CB_CUDA(cudaFuncSetAttribute(weight_grad_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         attr = true;
     }
-    int dev = 0, nsm = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const long long nChunks = (long long)((L.nI + WG_CH - 1) / WG_CH) * L.nJ * L.nK;
-    // a few CTAs per SM, each accumulating many chunks in tensor memory before its atomics
-    const long long g = std::min<long long>(nChunks, 4LL * nsm);
-    weight_grad_tc_kernel<<<(unsigned)(g > 0 ? g : 1), 128, smem, st>>>(L, x, dz, dW, db, err);
-    CB_CHECK_LAUNCH();
+    const long long most = weight_grad_ctas();
+    double* dbPart = reinterpret_cast<double*>(part + (size_t)most * WG_W);
+    for (int b = 0; b < n; b += CONV_MAX_JOBS) {
+        WgGroup g;
+        std::memset(&g, 0, sizeof(g));
+        g.n = std::min(CONV_MAX_JOBS, n - b);
+        long long chunks = 0;
+        for (int p = 0; p < g.n; ++p) {
+            const WgSpec& sp = specs[b + p];
+            g.L[p] = sp.L; g.x[p] = sp.x; g.dz[p] = sp.dz;
+            chunks += (long long)((sp.L.nI + WG_CH - 1) / WG_CH) * sp.L.nJ * sp.L.nK;
+            g.end[p] = chunks;
+        }
+        // four CTAs per SM at most; at least four chunks each, so that small lattices leave fewer partials
+        const long long ctas = std::max(1ll, std::min(most, chunks / 4));
+        weight_grad_tc_kernel<<<(unsigned)ctas, 128, smem, st>>>(g, part, dbPart, err);
+        weight_grad_sum_kernel<<<WG_W / 32 + 1, 256, 0, st>>>(part, dbPart, (int)ctas, grad, err);
+        CB_CHECK_LAUNCH();
+    }
     return 0;
 }
 

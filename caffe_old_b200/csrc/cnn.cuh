@@ -36,9 +36,16 @@ struct ConvSpec {
 int launch_conv3d_group(int epi, const ConvSpec* specs, int n, const __nv_bfloat16* wpack, const float* bias, int* err, cudaStream_t st,
                         const int* skip = nullptr);
 
-// Weight gradient of one layer on the tensor cores: dW[t][o][i] += sum_c x[c + off(t)][i] dz[c][o],
-// db[o] += sum_c dz[c][o] (FP32, accumulated into dW / db).
-int launch_weight_grad(const Lat& L, const __nv_bfloat16* x, const __nv_bfloat16* dz, float* dW, float* db, int* err, cudaStream_t st);
+// Weight gradient of one layer on the tensor cores over several lattices: grad = dW[t][o][i], then
+// db[o], with dW[t][o][i] += sum_c x[c + off(t)][i] dz[c][o], db[o] += sum_c dz[c][o] (FP32).
+// part: weight_grad_part_floats() floats of scratch.
+struct WgSpec {
+    Lat L;
+    const __nv_bfloat16* x;
+    const __nv_bfloat16* dz;
+};
+size_t weight_grad_part_floats();
+int launch_weight_grad_group(const WgSpec* specs, int n, float* grad, float* part, int* err, cudaStream_t st);
 
 // Device buffers of one network applied on one lattice.
 struct NetBuffers {
@@ -49,6 +56,7 @@ struct NetBuffers {
     __nv_bfloat16* wbwd;        // 4 x 27 x 512 bytes, transposed + flipped packing (backward data)
     float* params;              // NET_PARAMS (device master copy)
     float* grad;                // NET_PARAMS
+    float* wgPart;              // partial weight gradients of one launch
     float* y;                   // N: network output
     int* err;
 };
@@ -64,8 +72,9 @@ int net_forward_if(NetBuffers& nb, const int* skip, cudaStream_t st);
 // the forward passes of several networks that share one set of weights (nets[0]'s), one
 // launch per layer for all of them
 int net_forward_group_if(NetBuffers* const* nets, int n, const int* skip, cudaStream_t st);
-// backward for dL/dy (FP32, N): accumulates dL/dparams into nb.grad
-int net_backward(NetBuffers& nb, const float* dy, cudaStream_t st);
+// backward for dL/dy = scale[q] * dy[q] (FP32, N) of several networks that share one set of weights:
+// accumulates dL/dparams into nets[0]->grad; one launch per layer and pass for all of them
+int net_backward_group(NetBuffers* const* nets, const float* const* dy, const float* scale, int n, cudaStream_t st);
 // act[0] from a 2-channel FP32 input laid out [N][2]
 int net_pack_input2(NetBuffers& nb, const float* x2, cudaStream_t st);
 

@@ -1727,8 +1727,6 @@ int learned_alloc(LearnedWork& lw, const Lat& L, void* (*alloc)(size_t, void*), 
         Lat Lc = make_lat(c.n[0], c.n[1], c.n[2]);
         int rc = lw.nLev == 1 ? net_alloc(c.net, Lc, alloc, ctx) : net_alloc_shared(c.net, Lc, lw.lev[1].net, alloc, ctx);
         if (rc || net_alloc_shared(c.netNeg, Lc, lw.lev[1].net, alloc, ctx)) return 1;
-        c.w2 = static_cast<float*>(alloc(sizeof(float) * (size_t)c.N, ctx));
-        if (!c.w2) { set_error("learned-solver allocation failed"); return 1; }
         ++lw.nLev;
     }
     lw.weights = lw.nLev >= 2 ? &lw.lev[1].net : nullptr;
@@ -2055,11 +2053,6 @@ struct TrainScal {
     double s, coef, loss, loss_sum;
 };
 
-__global__ void half_split_kernel(long long n, float* a, float* b) {
-    long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (c < n) { float v = 0.5f * a[c]; a[c] = v; b[c] = -v; }
-}
-
 __global__ void __launch_bounds__(LB) train_scale_kernel(long long N, const float* b, const float* invD, const uint8_t* st, double* part) {
     double v[2] = {0., 0.};
     for (long long c = blockIdx.x * (long long)LB + threadIdx.x; c < N; c += (long long)gridDim.x * LB) {
@@ -2229,6 +2222,10 @@ int learned_train(LearnedWork& lw, const OpSym& A, const uint8_t* status, const 
             if (pair_forward(lw, Af, status, L, b, xs, NET_MODE_NETWORK, T, nullptr, st)) return 1;
             train_dz_kernel<<<G, 256, 0, st>>>(N, lw.e, status, T, inv_batch, lw.r);
             // adjoint chain: dL/dw_l = P_l^T dL/dw_(l-1) (into u_l), dL/dy_l = gain_l s dL/dw_l (into w_l)
+            NetBuffers* nets[2 * LEARN_MAX_LEVELS];
+            const float* dys[2 * LEARN_MAX_LEVELS];
+            float scale[2 * LEARN_MAX_LEVELS];
+            int nn = 0;
             for (int l = 1; l < lw.nLev; ++l) {
                 Level& c = lw.lev[l];
                 const Level& f = lw.lev[l - 1];
@@ -2236,10 +2233,12 @@ int learned_train(LearnedWork& lw, const OpSym& A, const uint8_t* status, const 
                                                                            c.u, c.w, c.gain, nullptr, nullptr, nullptr, 0.f, S);
                 if (l >= lw.netFrom && l <= lw.netTo) {
                     // y = (net(x) - net(-x)) / 2: the two evaluations get dL/dy / 2 and -dL/dy / 2
-                    half_split_kernel<<<grid_for(c.N, 256), 256, 0, st>>>(c.N, c.w, c.w2);
-                    if (net_backward(c.net, c.w, st) || net_backward(c.netNeg, c.w2, st)) return 1;
+                    nets[nn] = &c.net; dys[nn] = c.w; scale[nn++] = 0.5f;
+                    nets[nn] = &c.netNeg; dys[nn] = c.w; scale[nn++] = -0.5f;
                 }
             }
+            CB_CHECK_LAUNCH();
+            if (net_backward_group(nets, dys, scale, nn, st)) return 1;
         }
         loss_out_kernel<<<1, 32, 0, st>>>(T, hist, step, inv_batch);
         adam_kernel<<<grid_for(NET_PARAMS, 256), 256, 0, st>>>(NET_PARAMS, W.params, W.grad, mom, vel, lr, 0.9f, 0.999f, 1e-8f, step + 1);

@@ -45,13 +45,24 @@ __global__ void pack_input2_kernel(long long N, const float* __restrict__ x2, __
     dst[1] = reinterpret_cast<uint4*>(v)[1];
 }
 
-__global__ void pack_dy_kernel(long long N, const float* __restrict__ dy, __nv_bfloat16* gz) {
+// gz = (scale * dy, 0, ..., 0) of every job's cells
+struct PackJobs {
+    const float* dy[CONV_MAX_JOBS];
+    __nv_bfloat16* gz[CONV_MAX_JOBS];
+    float scale[CONV_MAX_JOBS];
+    long long end[CONV_MAX_JOBS];   // inclusive prefix sums of the cell counts
+    int n;
+};
+__global__ void pack_dy_kernel(const __grid_constant__ PackJobs g) {
     long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (c >= N) return;
+    if (c >= g.end[g.n - 1]) return;
+    int job = 0;
+    while (c >= g.end[job]) ++job;
+    if (job > 0) c -= g.end[job - 1];
     __align__(16) __nv_bfloat16 v[16];
-    v[0] = __float2bfloat16_rn(dy[c]);
+    v[0] = __float2bfloat16_rn(g.scale[job] * g.dy[job][c]);
     for (int q = 1; q < 16; ++q) v[q] = __float2bfloat16_rn(0.f);
-    uint4* dst = reinterpret_cast<uint4*>(gz + c * 16);
+    uint4* dst = reinterpret_cast<uint4*>(g.gz[job] + c * 16);
     dst[0] = reinterpret_cast<uint4*>(v)[0];
     dst[1] = reinterpret_cast<uint4*>(v)[1];
 }
@@ -67,9 +78,10 @@ int net_alloc(NetBuffers& nb, const Lat& L, void* (*alloc)(size_t, void*), void*
     nb.wbwd = static_cast<__nv_bfloat16*>(alloc((size_t)NET_LAYERS * 27 * 512, ctx));
     nb.params = static_cast<float*>(alloc(sizeof(float) * NET_PARAMS, ctx));
     nb.grad = static_cast<float*>(alloc(sizeof(float) * NET_PARAMS, ctx));
+    nb.wgPart = static_cast<float*>(alloc(sizeof(float) * weight_grad_part_floats(), ctx));
     nb.y = static_cast<float*>(alloc(sizeof(float) * (size_t)L.N, ctx));
     nb.err = static_cast<int*>(alloc(sizeof(int) * 4, ctx));
-    bool ok = nb.wfwd && nb.wbwd && nb.params && nb.grad && nb.y && nb.err;
+    bool ok = nb.wfwd && nb.wbwd && nb.params && nb.grad && nb.wgPart && nb.y && nb.err;
     for (int q = 0; q < 4; ++q) ok = ok && nb.act[q];
     for (int q = 0; q < 2; ++q) ok = ok && nb.gz[q];
     if (!ok) { set_error("network buffer allocation failed"); return 1; }
@@ -84,7 +96,7 @@ int net_alloc_shared(NetBuffers& nb, const Lat& L, const NetBuffers& owner, void
     for (int q = 0; q < 2; ++q) ok = ok && (nb.gz[q] = static_cast<__nv_bfloat16*>(alloc(actBytes, ctx)));
     ok = ok && (nb.y = static_cast<float*>(alloc(sizeof(float) * (size_t)L.N, ctx)));
     if (!ok) { set_error("network buffer allocation failed"); return 1; }
-    nb.wfwd = owner.wfwd; nb.wbwd = owner.wbwd; nb.params = owner.params; nb.grad = owner.grad; nb.err = owner.err;
+    nb.wfwd = owner.wfwd; nb.wbwd = owner.wbwd; nb.params = owner.params; nb.grad = owner.grad; nb.wgPart = owner.wgPart; nb.err = owner.err;
     return 0;
 }
 
@@ -131,21 +143,36 @@ int net_forward_group_if(NetBuffers* const* nets, int n, const int* skip, cudaSt
     return 0;
 }
 
-static int weight_grad(NetBuffers& nb, int l, const __nv_bfloat16* x, const __nv_bfloat16* dz, cudaStream_t st) {
-    float* g = nb.grad + (size_t)l * NET_LAYER_PARAMS;
-    return launch_weight_grad(nb.L, x, dz, g, g + 27 * 256, nb.err, st);
-}
-
-int net_backward(NetBuffers& nb, const float* dy, cudaStream_t st) {
-    const Lat& L = nb.L;
-    pack_dy_kernel<<<grid_for(L.N, 256), 256, 0, st>>>(L.N, dy, nb.gz[0]);
+int net_backward_group(NetBuffers* const* nets, const float* const* dy, const float* scale, int n, cudaStream_t st) {
+    if (n < 1) return 0;
+    NetBuffers& w = *nets[0];
+    for (int b = 0; b < n; b += CONV_MAX_JOBS) {
+        PackJobs g;
+        std::memset(&g, 0, sizeof(g));
+        g.n = n - b < CONV_MAX_JOBS ? n - b : CONV_MAX_JOBS;
+        long long cells = 0;
+        for (int p = 0; p < g.n; ++p) {
+            if (nets[b + p]->wfwd != w.wfwd) { set_error("grouped networks must share their weights"); return 1; }
+            g.dy[p] = dy[b + p]; g.gz[p] = nets[b + p]->gz[0]; g.scale[p] = scale[b + p];
+            cells += nets[b + p]->L.N;
+            g.end[p] = cells;
+        }
+        pack_dy_kernel<<<grid_for(cells, 256), 256, 0, st>>>(g);
+    }
     CB_CHECK_LAUNCH();
+    std::vector<WgSpec> wg((size_t)n);
+    std::vector<ConvSpec> cv((size_t)n);
     int a = 0;
     for (int l = 3; l >= 0; --l) {
-        if (weight_grad(nb, l, nb.act[l], nb.gz[a], st)) return 1;
+        for (int q = 0; q < n; ++q) { wg[q].L = nets[q]->L; wg[q].x = nets[q]->act[l]; wg[q].dz = nets[q]->gz[a]; }
+        if (launch_weight_grad_group(wg.data(), n, w.grad + (size_t)l * NET_LAYER_PARAMS, w.wgPart, w.err, st)) return 1;
         if (l == 0) break;
         // dL/dz of layer l-1 = (W_l^T applied to dz_l) where the layer's input was positive
-        if (launch_conv3d(L, 2, nb.gz[a], wb_of(nb, l), nullptr, nb.gz[a ^ 1], nullptr, nb.act[l], nb.err, st)) return 1;
+        for (int q = 0; q < n; ++q) {
+            cv[q].L = nets[q]->L; cv[q].in = nets[q]->gz[a]; cv[q].out_bf = nets[q]->gz[a ^ 1]; cv[q].out_f = nullptr;
+            cv[q].mask = nets[q]->act[l];
+        }
+        if (launch_conv3d_group(2, cv.data(), n, wb_of(w, l), nullptr, w.err, st)) return 1;
         a ^= 1;
     }
     return 0;
@@ -182,7 +209,10 @@ int run_host_net(int nI, int nJ, int nK, const float* params, const float* x2, c
     CB_CUDA(cudaMemcpy(dx2, x2, sizeof(float) * 2 * L.N, cudaMemcpyHostToDevice));
     if (dy) CB_CUDA(cudaMemcpy(ddy, dy, sizeof(float) * L.N, cudaMemcpyHostToDevice));
     if (net_pack_weights(nb, 0) || net_pack_input2(nb, dx2, 0) || net_forward(nb, 0)) return 1;
-    if (dy && net_backward(nb, ddy, 0)) return 1;
+    NetBuffers* const one[1] = {&nb};
+    const float* const ddys[1] = {ddy};
+    const float scale[1] = {1.f};
+    if (dy && net_backward_group(one, ddys, scale, 1, 0)) return 1;
     CB_CUDA(cudaDeviceSynchronize());
     int herr = 0;
     CB_CUDA(cudaMemcpy(&herr, nb.err, sizeof(int), cudaMemcpyDeviceToHost));
