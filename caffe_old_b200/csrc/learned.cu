@@ -145,14 +145,17 @@ __device__ __forceinline__ void totals_cg(const double* part, int nblk, int K, d
 }
 
 // after block_sums: true in every thread of the block that finished last (its partial and all
-// the others' are then in memory); that block resets the counter for the next kernel
+// the others' are then in memory); that block resets the counter for the next kernel.  The thread
+// that wrote the block's partials counts it in, release and acquire in one: a device-wide fence by every
+// thread of 2048 blocks had cost the 3.1M-cell product 13 of its 35 us.
 __device__ __forceinline__ bool last_block(unsigned* ctr) {
     __shared__ int amLast;
-    __threadfence();
+    if (threadIdx.x == 0) {
+        unsigned before;
+        asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(ctr) : "memory");
+        amLast = before == gridDim.x - 1;
+    }
     __syncthreads();
-    if (threadIdx.x == 0) amLast = atomicAdd(ctr, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (amLast) __threadfence();
     return amLast != 0;
 }
 
@@ -744,13 +747,27 @@ __device__ __forceinline__ void prolong4_ijk(const Dims3& fd, const Dims3& cd, c
 }
 
 // ---------------------------------------------------------------- coarse tail of the pyramid
-// The coarsest levels in one CTA (pyramid mode): u_lt = R u_(lt-1), with u_(lt-1) staged from global
-// memory into shared memory, u_(l+1) = R u_l, then w_last = gain u_last and
-// w_l = gain_l u_l + P w_(l+1) back up to lt, all in shared memory; u_l and w_l of every tail level
-// are written out.  It replaces 2 (levels - lt) launches of a few hundred cells each by one, with
-// the arithmetic of restrict_kernel and prolong_kernel in the same order.
-constexpr int TAIL_MAX_IN = 8192;       // cells of level lt-1 (staged)
-constexpr int TAIL_THREADS = 1024;
+// The coarsest levels in one thread-block cluster (levels that run no network): from the first level
+// lt of at most TAIL_MAX cells, u_lt = R u_(lt-1) and u_(l+1) = R u_l down to the coarsest, then
+// w_last = gain u_last, w_l = gain_l u_l + P w_(l+1) back up to lt, and to lt-1 where no network runs
+// there either.  Larger levels are dealt out over the cluster's blocks; once a level has at most
+// TAIL_OWN cells, every block works out the rest for itself in shared memory, so that the whole tail
+// takes about three cluster barriers.
+//
+// A launch of a few thousand cells costs its latency, 4 to 15 us: on the 192x128x128 pyramid this
+// kernel's TAIL_NEW us replace 31 (a restriction, a one-block tail from the level below, two
+// prolongations), twice per BiCGStab iteration of 290 us.
+//
+// Every value is formed as the kernels that these levels had before formed it, operation by operation
+// (written out with fused multiply-adds, so that it does not hang on what the compiler contracts): a
+// change in the last bit of the preconditioner moves an FP32 Krylov solve's result by as much as its
+// tolerance allows.  Hence the two orders of the first pair in a restriction's j and k passes: levels
+// below one of at most TAIL_PAIR cells multiply the first of the two first.
+constexpr int TAIL_MAX = 8192;          // cells of level lt
+constexpr int TAIL_MAX_IN = 65536;      // cells of level lt-1
+constexpr int TAIL_OWN = 256;           // cells of a level that every block works out for itself
+constexpr int TAIL_PAIR = 8192;         // cells of the level above: order of the first pair (see above)
+constexpr int TAIL_THREADS = 1024, TAIL_BLOCKS = 16;
 struct TailArgs {
     int n;                              // tail levels lt .. lt+n-1
     Dims3 d[LEARN_MAX_LEVELS + 1];      // d[0]: level lt-1; d[1..n]: the tail levels
@@ -758,34 +775,44 @@ struct TailArgs {
     const float* uin;                   // u of level lt-1
     float* u[LEARN_MAX_LEVELS];
     float* w[LEARN_MAX_LEVELS];
+    float* wFine;                       // w of level lt-1, or null: left to the caller
+    float gainFine;
 };
 
-__device__ __forceinline__ float tail_restrict_at(const float* fin, const Dims3& fd, const Dims3& cd, int I, int J, int K, float scale) {
+__device__ __forceinline__ float tail_sum4(const float (&w)[4], const float (&v)[4], bool firstRounded) {
+    const float s = firstRounded ? __fmaf_rn(w[1], v[1], __fmul_rn(w[0], v[0])) : __fmaf_rn(w[0], v[0], __fmul_rn(w[1], v[1]));
+    return __fmaf_rn(w[3], v[3], __fmaf_rn(w[2], v[2], s));
+}
+__device__ __forceinline__ float tail_blend(float a, float b) { return __fmaf_rn(0.75f, a, __fmul_rn(0.25f, b)); }
+
+// The 64 fine values a coarse cell draws on: offsets per direction, clamped to the lattice (a value
+// beyond it has weight zero), so that a row of four costs its loads and multiply-adds.
+__device__ __forceinline__ float tail_restrict_at(const float* fin, const Dims3& fd, const Dims3& cd, int I, int J, int K, float scale,
+                                                  bool pair) {
+    float wi[4], wj[4], wk[4];
+    int oi[4], oj[4], ok[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        wi[m] = rweight_in(2 * I - 1 + m, fd.n0, I, cd.n0);
+        wj[m] = rweight_in(2 * J - 1 + m, fd.n1, J, cd.n1);
+        wk[m] = rweight_in(2 * K - 1 + m, fd.n2, K, cd.n2);
+        oi[m] = pclamp(2 * I - 1 + m, fd.n0);
+        oj[m] = pclamp(2 * J - 1 + m, fd.n1) * fd.n0;
+        ok[m] = pclamp(2 * K - 1 + m, fd.n2) * fd.n0 * fd.n1;
+    }
     float t2[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-        const int fk = 2 * K - 1 + c;
         float t1[4];
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
-            const int fj = 2 * J - 1 + b;
-            float v[4];
-#pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                const int fi = 2 * I - 1 + a;
-                const bool in = fi >= 0 && fi < fd.n0 && fj >= 0 && fj < fd.n1 && fk >= 0 && fk < fd.n2;
-                v[a] = in ? fin[((unsigned)fk * (unsigned)fd.n1 + (unsigned)fj) * (unsigned)fd.n0 + (unsigned)fi] : 0.f;
-            }
-            t1[b] = rweight_in(2 * I - 1, fd.n0, I, cd.n0) * v[0] + rweight_in(2 * I, fd.n0, I, cd.n0) * v[1] +
-                    rweight_in(2 * I + 1, fd.n0, I, cd.n0) * v[2] + rweight_in(2 * I + 2, fd.n0, I, cd.n0) * v[3];
+            const float* row = fin + (ok[c] + oj[b]);
+            const float v[4] = {row[oi[0]], row[oi[1]], row[oi[2]], row[oi[3]]};
+            t1[b] = tail_sum4(wi, v, false);
         }
-        t2[c] = rweight_in(2 * J - 1, fd.n1, J, cd.n1) * t1[0] + rweight_in(2 * J, fd.n1, J, cd.n1) * t1[1] +
-                rweight_in(2 * J + 1, fd.n1, J, cd.n1) * t1[2] + rweight_in(2 * J + 2, fd.n1, J, cd.n1) * t1[3];
+        t2[c] = tail_sum4(wj, t1, pair);
     }
-    float acc = rweight_in(2 * K - 1, fd.n2, K, cd.n2) * t2[0] + rweight_in(2 * K, fd.n2, K, cd.n2) * t2[1] +
-                rweight_in(2 * K + 1, fd.n2, K, cd.n2) * t2[2] + rweight_in(2 * K + 2, fd.n2, K, cd.n2) * t2[3];
-    acc *= scale;
-    return acc;
+    return __fmul_rn(tail_sum4(wk, t2, pair), scale);
 }
 
 // prolong_at on a shared-memory coarse array (plain loads), the same blend order
@@ -801,48 +828,102 @@ __device__ __forceinline__ float tail_prolong_at(const Dims3& fd, const Dims3& c
     const unsigned sJ = (unsigned)cd.n0, sK = (unsigned)cd.n0 * (unsigned)cd.n1;
     auto row = [&](int K, int J) {
         const float* w = wc + (unsigned)K * sK + (unsigned)J * sJ;
-        return 0.75f * w[I0] + 0.25f * w[I1];
+        return tail_blend(w[I0], w[I1]);
     };
-    float k0 = 0.75f * row(K0, J0) + 0.25f * row(K0, J1);
-    float k1 = 0.75f * row(K1, J0) + 0.25f * row(K1, J1);
-    return 0.75f * k0 + 0.25f * k1;
+    const float k0 = tail_blend(row(K0, J0), row(K0, J1));
+    const float k1 = tail_blend(row(K1, J0), row(K1, J1));
+    return tail_blend(k0, k1);
 }
 
-__global__ void __launch_bounds__(TAIL_THREADS) coarse_tail_kernel(const __grid_constant__ TailArgs a, const Scal* S) {
-    if (S && S->done) return;
+// out = gain y + P wc for the cells of lattice fd, dealt out from `from` in steps of `step`; two cells
+// fi, fi + 1 (fi even) at a time where rows are even: they draw on coarse columns F-1, F, F+1 (F = fi / 2)
+// of the same four rows
+__device__ __forceinline__ void tail_prolong(const Dims3& fd, const Dims3& cd, const float* wc, const float* y, float gain, float* out, int from,
+                                             int step) {
+    const int N = fd.n0 * fd.n1 * fd.n2;
+    if (fd.n0 & 1) {
+        for (int c = from; c < N; c += step) out[c] = __fmaf_rn(gain, y[c], tail_prolong_at(fd, cd, wc, c));
+        return;
+    }
+    const unsigned half = (unsigned)fd.n0 >> 1;
+    for (int h = from; h < N / 2; h += step) {
+        const unsigned t = (unsigned)h / half, F = (unsigned)h - t * half, uk = t / (unsigned)fd.n1;
+        const int fk = (int)uk, fj = (int)(t - uk * (unsigned)fd.n1);
+        const int J0 = fj >> 1, J1 = pclamp((fj & 1) ? J0 + 1 : J0 - 1, cd.n1);
+        const int K0 = fk >> 1, K1 = pclamp((fk & 1) ? K0 + 1 : K0 - 1, cd.n2);
+        const int A0 = pclamp((int)F - 1, cd.n0), A2 = pclamp((int)F + 1, cd.n0), sK = cd.n0 * cd.n1;
+        float lo[4], hi[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const float* row = wc + ((r & 2 ? K1 : K0) * sK + (r & 1 ? J1 : J0) * cd.n0);
+            const float x0 = row[A0], x1 = row[F], x2 = row[A2];
+            lo[r] = tail_blend(x1, x0);
+            hi[r] = tail_blend(x1, x2);
+        }
+        out[2 * h] = __fmaf_rn(gain, y[2 * h], tail_blend(tail_blend(lo[0], lo[1]), tail_blend(lo[2], lo[3])));
+        out[2 * h + 1] = __fmaf_rn(gain, y[2 * h + 1], tail_blend(tail_blend(hi[0], hi[1]), tail_blend(hi[2], hi[3])));
+    }
+}
+
+__global__ void __cluster_dims__(TAIL_BLOCKS, 1, 1) __launch_bounds__(TAIL_THREADS) coarse_tail_kernel(const __grid_constant__ TailArgs a,
+                                                                                                  const Scal* S) {
+    if (S && S->done) return;   // uniform across the cluster
     extern __shared__ float tsm[];
-    long long off[LEARN_MAX_LEVELS + 1];
-    long long total = 0;
-    for (int l = 0; l <= a.n; ++l) {
-        off[l] = total;
-        total += (long long)a.d[l].n0 * a.d[l].n1 * a.d[l].n2;
-    }
-    float* U = tsm;                    // u of levels lt-1 .. lt+n-1, packed
-    float* W = tsm + total - off[1];   // w of the tail levels (the same offsets; nothing for lt-1)
-    const long long n0 = off[1];
-    for (long long c = threadIdx.x; c < n0; c += blockDim.x) U[c] = a.uin[c];
-    __syncthreads();
-    for (int l = 1; l <= a.n; ++l) {
+    auto barrier = [] {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    };
+    auto cells = [&](int l) { return a.d[l].n0 * a.d[l].n1 * a.d[l].n2; };
+    const int all = blockIdx.x * TAIL_THREADS + threadIdx.x, allStep = TAIL_BLOCKS * TAIL_THREADS;
+    auto down = [&](const float* fin, int l, int c) {
         const Dims3 fd = a.d[l - 1], cd = a.d[l];
-        const long long N = (long long)cd.n0 * cd.n1 * cd.n2;
-        for (long long c = threadIdx.x; c < N; c += blockDim.x) {
-            const int I = (int)(c % cd.n0), J = (int)((c / cd.n0) % cd.n1), K = (int)(c / ((long long)cd.n0 * cd.n1));
-            const float v = tail_restrict_at(U + off[l - 1], fd, cd, I, J, K, a.rscale[l - 1]);
-            U[off[l] + c] = v;
-            a.u[l - 1][c] = v;
+        const unsigned t = (unsigned)c / (unsigned)cd.n0, K = t / (unsigned)cd.n1;
+        return tail_restrict_at(fin, fd, cd, c - (int)(t * (unsigned)cd.n0), (int)(t - K * (unsigned)cd.n1), (int)K, a.rscale[l - 1],
+                                fd.n0 * fd.n1 * fd.n2 <= TAIL_PAIR);
+    };
+    // down: levels 1 .. nd are dealt out over the blocks
+    int nd = 0;
+    do {
+        ++nd;
+        const float* fin = nd == 1 ? a.uin : a.u[nd - 2];
+        const int N = cells(nd);
+        for (int c = all; c < N; c += allStep) a.u[nd - 1][c] = down(fin, nd, c);
+        barrier();
+    } while (nd < a.n && cells(nd + 1) > TAIL_OWN);
+    // the rest in every block's shared memory: u of levels nd .. n, then w of the same
+    int total = 0;
+    for (int l = nd; l <= a.n; ++l) total += cells(l);
+    for (int c = threadIdx.x; c < cells(nd); c += TAIL_THREADS) tsm[c] = a.u[nd - 1][c];
+    __syncthreads();
+    for (int l = nd + 1, o = 0; l <= a.n; ++l) {
+        float* u = tsm + o + cells(l - 1);
+        for (int c = threadIdx.x; c < cells(l); c += TAIL_THREADS) {
+            const float v = down(tsm + o, l, c);
+            u[c] = v;
+            if (blockIdx.x == 0) a.u[l - 1][c] = v;
         }
+        o += cells(l - 1);
         __syncthreads();
     }
-    for (int l = a.n; l >= 1; --l) {
-        const Dims3 fd = a.d[l];
-        const long long N = (long long)fd.n0 * fd.n1 * fd.n2;
-        for (long long c = threadIdx.x; c < N; c += blockDim.x) {
-            float v = a.gain[l - 1] * 1.f * U[off[l] + c];
-            if (l < a.n) v += tail_prolong_at(fd, a.d[l + 1], W + off[l + 1], c);
-            W[off[l] + c] = v;
-            a.w[l - 1][c] = v;
-        }
+    for (int l = a.n, o = total; l >= nd; --l) {
+        o -= cells(l);
+        float *u = tsm + o, *w = u + total;
+        if (l == a.n)
+            for (int c = threadIdx.x; c < cells(l); c += TAIL_THREADS) w[c] = __fmul_rn(a.gain[l - 1], u[c]);
+        else
+            tail_prolong(a.d[l], a.d[l + 1], w + cells(l), u, a.gain[l - 1], w, threadIdx.x, TAIL_THREADS);
         __syncthreads();
+        if (blockIdx.x == 0)
+            for (int c = threadIdx.x; c < cells(l); c += TAIL_THREADS) a.w[l - 1][c] = w[c];
+    }
+    // up again over the blocks, from the w of level nd in shared memory
+    const float* wc = tsm + total;
+    for (int l = nd - 1; l >= (a.wFine ? 0 : 1); --l) {
+        const float* y = l > 0 ? a.u[l - 1] : a.uin;
+        float* w = l > 0 ? a.w[l - 1] : a.wFine;
+        tail_prolong(a.d[l], a.d[l + 1], wc, y, l > 0 ? a.gain[l - 1] : a.gainFine, w, all, allStep);
+        if (l > (a.wFine ? 0 : 1)) barrier();
+        wc = w;
     }
 }
 
@@ -1575,16 +1656,14 @@ Dims3 dims_of(const Level& l) { return Dims3{l.n[0], l.n[1], l.n[2]}; }
 int apply_levels(LearnedWork& lw, const float* rfine, const uint8_t* status, int mode, Scal* S, cudaStream_t st, const float* ufine = nullptr) {
     if (mode == NET_MODE_JACOBI || lw.nLev < 2) return 0;
     auto netAt = [&](int l) { return mode == NET_MODE_NETWORK && l >= lw.netFrom && l <= lw.netTo; };
-    // the coarse tail: from the first level lt >= 2 whose finer neighbour has at most TAIL_MAX_IN
-    // cells and from which on no level runs the network, one kernel does the rest of the pyramid
+    // the coarse tail: from the first level lt >= 2 of at most TAIL_MAX cells (TAIL_MAX_IN on the level
+    // above) on, if no level from there on runs the network, one kernel does the rest of the pyramid
     int lt = lw.nLev;
-    long long tailCells = 0;   // u and w of the tail levels, in shared memory with the staged input
     for (int l = lw.nLev - 1; l >= 2; --l) {
-        if (netAt(l) || lw.lev[l - 1].N > TAIL_MAX_IN) break;
-        if ((size_t)(lw.lev[l - 1].N + 2 * (tailCells + lw.lev[l].N)) * sizeof(float) > 48 * 1024) break;
-        tailCells += lw.lev[l].N;
+        if (netAt(l) || lw.lev[l].N > TAIL_MAX || lw.lev[l - 1].N > TAIL_MAX_IN) break;
         lt = l;
     }
+    const bool tailFine = lt < lw.nLev && !netAt(lt - 1);   // the tail also prolongs to level lt-1
     for (int l = 1; l < lt; ++l) {
         Level& c = lw.lev[l];
         const Level& f = lw.lev[l - 1];
@@ -1623,7 +1702,9 @@ int apply_levels(LearnedWork& lw, const float* rfine, const uint8_t* status, int
         ta.n = lw.nLev - lt;
         ta.d[0] = dims_of(lw.lev[lt - 1]);
         ta.uin = lw.lev[lt - 1].u;
-        long long cells = lw.lev[lt - 1].N;
+        ta.wFine = tailFine ? lw.lev[lt - 1].w : nullptr;
+        ta.gainFine = lw.lev[lt - 1].gain;
+        long long cells = 0, held = 0;
         for (int q = 0; q < ta.n; ++q) {
             Level& c = lw.lev[lt + q];
             ta.d[q + 1] = dims_of(c);
@@ -1631,12 +1712,16 @@ int apply_levels(LearnedWork& lw, const float* rfine, const uint8_t* status, int
             ta.gain[q] = c.gain;
             ta.u[q] = c.u;
             ta.w[q] = c.w;
-            cells += 2 * c.N;
+            cells += q > 0 && lw.lev[lt + q].N <= TAIL_OWN ? 2 * c.N : 0;
+            // the last level dealt out is held as well
+            if (c.N > TAIL_OWN || q == 0) held = c.N;
         }
-        coarse_tail_kernel<<<1, TAIL_THREADS, sizeof(float) * (size_t)cells, st>>>(ta, S);
+        static const cudaError_t attr = cudaFuncSetAttribute(coarse_tail_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        CB_CUDA(attr);
+        coarse_tail_kernel<<<TAIL_BLOCKS, TAIL_THREADS, sizeof(float) * (size_t)(cells + 2 * held), st>>>(ta, S);
         CB_CHECK_LAUNCH();
     }
-    for (int l = lt - 1; l >= 1; --l) {
+    for (int l = tailFine ? lt - 2 : lt - 1; l >= 1; --l) {
         Level& f = lw.lev[l];
         const bool top = l + 1 >= lw.nLev;
         const float* y = netAt(l) ? f.net.y : f.u;
