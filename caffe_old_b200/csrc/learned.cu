@@ -159,6 +159,35 @@ __device__ __forceinline__ bool last_block(unsigned* ctr) {
     return amLast != 0;
 }
 
+// Programmatic dependent launch: a kernel of the inner iteration reads nothing before the previous
+// kernel's writes are complete (pdl_wait, first thing), and lets the next one's blocks be placed before
+// its own have all left (pdl_next): the small kernels of the coarse levels at once, the sweeps over the
+// cell lattice after their last load, since blocks that only wait took the places of blocks with
+// work to do (the p' solve on 384x256x256 ran 343 ms that way, 336 without dependent launches and 328
+// so).  About twenty kernels make an iteration; without it each pays the launch and the ramp of its
+// first blocks: a learned step on 192x128x128 took 286 ms, now 270.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_start() {
+    pdl_next();
+    pdl_wait();
+}
+template <class... P, class... A>
+int launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    CB_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+    return 0;
+}
+
 inline int nblocks(long long N) {
     long long b = (N + LB - 1) / LB;
     return (int)(b < MAXP ? b : MAXP);
@@ -291,6 +320,7 @@ constexpr int RFI = 2 * RCI + 2, RFJ = 2 * RCJ + 2, RFK = 2 * RCK + 2;
 __global__ void __launch_bounds__(256) restrict_kernel(Dims3 fd, Dims3 cd, const float* fin, const float* invD, const uint8_t* st,
                                                        float scale, float* out, float* out2, float mul2, __nv_bfloat16* act0,
                                                        __nv_bfloat16* act0n, const float* maskc, float chan, const Scal* S) {
+    pdl_start();
     if (S && S->done) return;
     __shared__ __align__(16) float s0[RFK][RFJ][RFI];
     __shared__ float t1[RFK][RFJ][RCI];
@@ -451,6 +481,7 @@ struct RestrictMaps {
 template <bool PRE>
 __global__ void __launch_bounds__(RT_THREADS, 2) restrict_tma_kernel(const __grid_constant__ RestrictMaps maps, Dims3 fd, Dims3 cd, int hasSt,
                                                                   float scale, float* out, int* err, const Scal* S) {
+    pdl_start();
     constexpr int STAGE = PRE ? RT_F_BYTES : RT_STAGE_BYTES;
     constexpr int NS = PRE ? 3 : 2;   // stages: tiles in flight ahead of the one being reduced = NS - 1
     if (S && S->done) return;
@@ -647,10 +678,10 @@ int launch_restrict_tma(const Dims3& fd, const Dims3& cd, const float* fin, cons
     const int sms = nsm > 0 ? nsm : 148;
     if (pre) {
         const int grid = (int)std::min<long long>(T, 2LL * sms);   // two CTAs per SM
-        restrict_tma_kernel<true><<<grid, RT_THREADS, smemPre, stream>>>(maps, fd, cd, 0, scale, out, err, S);
+        if (launch_pdl(restrict_tma_kernel<true>, dim3(grid), dim3(RT_THREADS), smemPre, stream, maps, fd, cd, 0, scale, out, err, S)) return 1;
     } else {
         const int grid = (int)std::min<long long>(T, sms);
-        restrict_tma_kernel<false><<<grid, RT_THREADS, smemFull, stream>>>(maps, fd, cd, st ? 1 : 0, scale, out, err, S);
+        if (launch_pdl(restrict_tma_kernel<false>, dim3(grid), dim3(RT_THREADS), smemFull, stream, maps, fd, cd, st ? 1 : 0, scale, out, err, S)) return 1;
     }
     CB_CHECK_LAUNCH();
     return 0;
@@ -867,6 +898,7 @@ __device__ __forceinline__ void tail_prolong(const Dims3& fd, const Dims3& cd, c
 
 __global__ void __cluster_dims__(TAIL_BLOCKS, 1, 1) __launch_bounds__(TAIL_THREADS) coarse_tail_kernel(const __grid_constant__ TailArgs a,
                                                                                                   const Scal* S) {
+    pdl_start();
     if (S && S->done) return;   // uniform across the cluster
     extern __shared__ float tsm[];
     auto barrier = [] {
@@ -931,6 +963,7 @@ __global__ void __cluster_dims__(TAIL_BLOCKS, 1, 1) __launch_bounds__(TAIL_THREA
 // network term is odd: y <- (y - yn) / 2 (yn = the network applied to the negated input)
 __global__ void __launch_bounds__(256) prolong_kernel(Dims3 fd, Dims3 cd, const float* wc, const float* y, const float* yn, int ydiv,
                                                       float gain, float* out, const Scal* S) {
+    pdl_start();
     if (S->done) return;
     long long Nf = (long long)fd.n0 * fd.n1 * fd.n2;
     long long f = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -947,6 +980,7 @@ __global__ void __launch_bounds__(256) prolong_kernel(Dims3 fd, Dims3 cd, const 
 // every value formed as prolong_kernel forms it
 __global__ void __launch_bounds__(256) prolong4_kernel(Dims3 fd, Dims3 cd, const float* wc, const float* y, const float* yn, int ydiv,
                                                        float gain, float* out, const Scal* S) {
+    pdl_start();
     if (S->done) return;
     const long long NQ = ((long long)fd.n0 * fd.n1 * fd.n2) >> 2;
     const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -1160,6 +1194,7 @@ __device__ __forceinline__ void fin_update(const double* t, Scal* S, int max_ite
 // p = r + beta (p - omega v); partial sum of (D^-1 p)^2 over active cells (scale of M(p))
 __global__ void __launch_bounds__(LB) bs_dir_kernel(long long N, const float* r, const float* v, const float* invD, const uint8_t* st,
                                                     float* p, double* part, Scal* S, unsigned* ctr, float* uo) {
+    pdl_wait();
     if (S->done) return;
     const float be = (float)S->beta, om = (float)S->omega;
     const long long T = (long long)gridDim.x * LB, t0 = blockIdx.x * (long long)LB + threadIdx.x, NQ = N >> 2;
@@ -1184,6 +1219,7 @@ __global__ void __launch_bounds__(LB) bs_dir_kernel(long long N, const float* r,
         if (is_active(st, c)) { double u = (double)__ldg(invD + c) * pv; a[0] += u * u; }
         if (uo) uo[c] = is_active(st, c) ? __ldg(invD + c) * pv : 0.f;
     }
+    pdl_next();
     block_sums(a, 1, part);
     if (ctr && last_block(ctr)) {
         double t[1];
@@ -1200,6 +1236,7 @@ __global__ void scale_finish(const double* part, int nblk, Scal* S) {
 // y = M(x) on the cell lattice: D^-1 x + P w_1 on active cells, D^-1 x on ghost rows, 0 on inactive cells
 __global__ void __launch_bounds__(LB) bs_z_kernel(long long N, Dims3 fd, Dims3 cd, const float* x, const float* invD, const uint8_t* st,
                                                   const float* w1, float* y, const Scal* S) {
+    pdl_wait();
     if (S->done) return;
     const long long T = (long long)gridDim.x * LB, t0 = blockIdx.x * (long long)LB + threadIdx.x, NQ = N >> 2;
     // lattice coordinates of cell 4q, stepped with the loop (no division inside it)
@@ -1245,6 +1282,7 @@ __global__ void __launch_bounds__(LB) bs_z_kernel(long long N, Dims3 fd, Dims3 c
         }
         y[c] = zv;
     }
+    pdl_next();
 }
 // A x for the 4 consecutive cells 4q .. 4q+3 (nI and nI*nJ multiples of 4, so every neighbouring
 // group of 4 is 16-byte aligned): 14 loads for the 4 rows instead of 14 per row.  The west /
@@ -1276,6 +1314,7 @@ __device__ __forceinline__ void spmv4(const OpSymF32& A, const float* x, long lo
 template <bool V4>
 __global__ void __launch_bounds__(LB, 5) bs_spmv_kernel(OpSymF32 A, long long N, const float* x, float* out, const float* a1, const float* b2,
                                                      double* part, Scal* S, unsigned* ctr) {
+    pdl_wait();
     if (S->done) return;
     double a[2] = {0., 0.};
     long long c0 = 0;
@@ -1305,6 +1344,7 @@ __global__ void __launch_bounds__(LB, 5) bs_spmv_kernel(OpSymF32 A, long long N,
         if (b2) { a[0] += (double)b2[c] * y; a[1] += (double)y * y; }
         else a[0] += (double)a1[c] * y;
     }
+    pdl_next();
     block_sums(a, b2 ? 2 : 1, part);
     if (ctr && last_block(ctr)) {
         double t[2];
@@ -1319,6 +1359,7 @@ __global__ void __launch_bounds__(LB, 5) bs_spmv_kernel(OpSymF32 A, long long N,
 // s = r - alpha v; partial sum of (D^-1 s)^2 over active cells
 __global__ void __launch_bounds__(LB) bs_s_kernel(long long N, const float* r, const float* v, const float* invD, const uint8_t* st, float* s,
                                                   double* part, Scal* S, unsigned* ctr, float* uo) {
+    pdl_wait();
     if (S->done) return;
     const float al = (float)S->alpha;
     const long long T = (long long)gridDim.x * LB, t0 = blockIdx.x * (long long)LB + threadIdx.x, NQ = N >> 2;
@@ -1343,6 +1384,7 @@ __global__ void __launch_bounds__(LB) bs_s_kernel(long long N, const float* r, c
         if (is_active(st, c)) { double u = (double)__ldg(invD + c) * sv; a[0] += u * u; }
         if (uo) uo[c] = is_active(st, c) ? __ldg(invD + c) * sv : 0.f;
     }
+    pdl_next();
     block_sums(a, 1, part);
     if (ctr && last_block(ctr)) {
         double t[1];
@@ -1353,6 +1395,7 @@ __global__ void __launch_bounds__(LB) bs_s_kernel(long long N, const float* r, c
 // e += alpha ph + omega sh; r = s - omega t; partials ||r||^2, (rhat, r)
 __global__ void __launch_bounds__(LB) bs_update_kernel(long long N, float* e, float* r, const float* ph, const float* sh, const float* s,
                                                        const float* t, const float* rh, double* part, Scal* S, unsigned* ctr, int max_iters) {
+    pdl_wait();
     if (S->done) return;
     const float al = (float)S->alpha, om = (float)S->omega;
     const long long T = (long long)gridDim.x * LB, t0 = blockIdx.x * (long long)LB + threadIdx.x, NQ = N >> 2;
@@ -1377,6 +1420,7 @@ __global__ void __launch_bounds__(LB) bs_update_kernel(long long N, float* e, fl
         a[0] += (double)rn * rn;
         a[1] += (double)rh[c] * rn;
     }
+    pdl_next();
     block_sums(a, 2, part);
     if (ctr && last_block(ctr)) {
         double tt[2];
@@ -1682,10 +1726,10 @@ int apply_levels(LearnedWork& lw, const float* rfine, const uint8_t* status, int
             if (launch_restrict_tma(dims_of(f), dims_of(c), f.u, nullptr, nullptr, c.rscale, c.u, lw.rtErr, S, st)) return 1;
             continue;
         }
-        restrict_kernel<<<restrict_grid(dims_of(c)), 256, 0, st>>>(dims_of(f), dims_of(c), l == 1 ? rfine : f.u, l == 1 ? lw.invD : nullptr,
+        if (launch_pdl(restrict_kernel, dim3(restrict_grid(dims_of(c))), dim3(256), 0, st, dims_of(f), dims_of(c), l == 1 ? rfine : f.u, l == 1 ? lw.invD : nullptr,
                                                                    l == 1 ? status : nullptr, c.rscale, c.u, nullptr, 0.f,
                                                                    netAt(l) ? c.net.act[0] : nullptr, netAt(l) ? c.netNeg.act[0] : nullptr,
-                                                                   c.mask, c.chan, S);
+                                                                   c.mask, c.chan, S)) return 1;
     }
     CB_CHECK_LAUNCH();
     // every network level and both signs of the odd form: one grouped launch per layer
@@ -1718,7 +1762,7 @@ int apply_levels(LearnedWork& lw, const float* rfine, const uint8_t* status, int
         }
         static const cudaError_t attr = cudaFuncSetAttribute(coarse_tail_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         CB_CUDA(attr);
-        coarse_tail_kernel<<<TAIL_BLOCKS, TAIL_THREADS, sizeof(float) * (size_t)(cells + 2 * held), st>>>(ta, S);
+        if (launch_pdl(coarse_tail_kernel, dim3(TAIL_BLOCKS), dim3(TAIL_THREADS), sizeof(float) * (size_t)(cells + 2 * held), st, ta, S)) return 1;
         CB_CHECK_LAUNCH();
     }
     for (int l = tailFine ? lt - 2 : lt - 1; l >= 1; --l) {
@@ -1727,13 +1771,10 @@ int apply_levels(LearnedWork& lw, const float* rfine, const uint8_t* status, int
         const float* y = netAt(l) ? f.net.y : f.u;
         const float* yn = netAt(l) ? f.netNeg.y : nullptr;
         auto a16 = [](const void* p) { return ((uintptr_t)p & 15u) == 0; };
-        if ((f.N & 3) == 0 && a16(y) && a16(f.w) && (!yn || a16(yn)))
-            prolong4_kernel<<<grid_for(f.N / 4, 256), 256, 0, st>>>(dims_of(f), top ? dims_of(f) : dims_of(lw.lev[l + 1]),
-                                                                    top ? nullptr : lw.lev[l + 1].w, y, yn, netAt(l) ? 0 : 1, f.gain,
-                                                                    f.w, S);
-        else
-            prolong_kernel<<<grid_for(f.N, 256), 256, 0, st>>>(dims_of(f), top ? dims_of(f) : dims_of(lw.lev[l + 1]),
-                                                               top ? nullptr : lw.lev[l + 1].w, y, yn, netAt(l) ? 0 : 1, f.gain, f.w, S);
+        const bool quads = (f.N & 3) == 0 && a16(y) && a16(f.w) && (!yn || a16(yn));
+        if (launch_pdl(quads ? prolong4_kernel : prolong_kernel, dim3(grid_for(quads ? f.N / 4 : f.N, 256)), dim3(256), 0, st, dims_of(f),
+                       top ? dims_of(f) : dims_of(lw.lev[l + 1]), top ? nullptr : lw.lev[l + 1].w, y, yn, netAt(l) ? 0 : 1, f.gain, f.w, S))
+            return 1;
     }
     CB_CHECK_LAUNCH();
     return 0;
@@ -1747,9 +1788,9 @@ int level_masks(LearnedWork& lw, const uint8_t* status, cudaStream_t st) {
     for (int l = 1; l < lw.nLev; ++l) {
         Level& c = lw.lev[l];
         const Level& f = lw.lev[l - 1];
-        restrict_kernel<<<restrict_grid(dims_of(c)), 256, 0, st>>>(dims_of(f), dims_of(c), l == 1 ? nullptr : f.mask, nullptr,
+        if (launch_pdl(restrict_kernel, dim3(restrict_grid(dims_of(c))), dim3(256), 0, st, dims_of(f), dims_of(c), l == 1 ? nullptr : f.mask, nullptr,
                                                                    l == 1 ? status : nullptr, c.rscale, c.mask, nullptr, 0.f, nullptr,
-                                                                   nullptr, nullptr, 0.f, nullptr);
+                                                                   nullptr, nullptr, 0.f, nullptr)) return 1;
     }
     CB_CHECK_LAUNCH();
     lw.masksReady = true;
@@ -1931,7 +1972,7 @@ int learned_solve(LearnedWork& lw, const OpSym& A, const uint8_t* status, const 
                     scale_partial_kernel<<<nb, LB, 0, st>>>(N, vj, lw.invD, status, lw.part, S, lw.u1);
                     scale_finish<<<1, LB, 0, st>>>(lw.part, nb, S);
                     if (apply_levels(lw, vj, status, mode, S, st, lw.u1)) return 1;
-                    bs_z_kernel<<<nb, LB, 0, st>>>(N, fd, cd, vj, lw.invD, status, w1, zj, S);
+                    if (launch_pdl(bs_z_kernel, dim3(nb), dim3(LB), 0, st, N, fd, cd, vj, lw.invD, status, w1, zj, S)) return 1;
                     if (v4) fg_spmv_kernel<true><<<nb, LB, 0, st>>>(Af, N, zj, lw.t, S);
                     else fg_spmv_kernel<false><<<nb, LB, 0, st>>>(Af, N, zj, lw.t, S);
                     // classical Gram-Schmidt with one re-orthogonalisation (CGS2): FP32 vectors lose
@@ -1980,17 +2021,15 @@ int learned_solve(LearnedWork& lw, const OpSym& A, const uint8_t* status, const 
                         cur ^= 1;
                     } else {
                         // p = p[0], v = q[0], ph = p[1], sh = q[1], s = z, t = t
-                        bs_dir_kernel<<<nb, LB, 0, st>>>(N, lw.r, lw.q[0], lw.invD, status, lw.p[0], lw.part, S, lw.ctr, lw.u1);
+                        if (launch_pdl(bs_dir_kernel, dim3(nb), dim3(LB), 0, st, N, lw.r, lw.q[0], lw.invD, status, lw.p[0], lw.part, S, lw.ctr, lw.u1)) return 1;
                         if (apply_levels(lw, lw.p[0], status, mode, S, st, lw.u1)) return 1;
-                        bs_z_kernel<<<nb, LB, 0, st>>>(N, fd, cd, lw.p[0], lw.invD, status, w1, lw.p[1], S);
-                        if (v4) bs_spmv_kernel<true><<<nb, LB, 0, st>>>(Af, N, lw.p[1], lw.q[0], lw.rh, nullptr, lw.part, S, lw.ctr);
-                        else bs_spmv_kernel<false><<<nb, LB, 0, st>>>(Af, N, lw.p[1], lw.q[0], lw.rh, nullptr, lw.part, S, lw.ctr);
-                        bs_s_kernel<<<nb, LB, 0, st>>>(N, lw.r, lw.q[0], lw.invD, status, lw.z, lw.part, S, lw.ctr, lw.u1);
+                        if (launch_pdl(bs_z_kernel, dim3(nb), dim3(LB), 0, st, N, fd, cd, lw.p[0], lw.invD, status, w1, lw.p[1], S)) return 1;
+                        if (launch_pdl(v4 ? bs_spmv_kernel<true> : bs_spmv_kernel<false>, dim3(nb), dim3(LB), 0, st, Af, N, lw.p[1], lw.q[0], lw.rh, nullptr, lw.part, S, lw.ctr)) return 1;
+                        if (launch_pdl(bs_s_kernel, dim3(nb), dim3(LB), 0, st, N, lw.r, lw.q[0], lw.invD, status, lw.z, lw.part, S, lw.ctr, lw.u1)) return 1;
                         if (apply_levels(lw, lw.z, status, mode, S, st, lw.u1)) return 1;
-                        bs_z_kernel<<<nb, LB, 0, st>>>(N, fd, cd, lw.z, lw.invD, status, w1, lw.q[1], S);
-                        if (v4) bs_spmv_kernel<true><<<nb, LB, 0, st>>>(Af, N, lw.q[1], lw.t, nullptr, lw.z, lw.part, S, lw.ctr);
-                        else bs_spmv_kernel<false><<<nb, LB, 0, st>>>(Af, N, lw.q[1], lw.t, nullptr, lw.z, lw.part, S, lw.ctr);
-                        bs_update_kernel<<<nb, LB, 0, st>>>(N, lw.e, lw.r, lw.p[1], lw.q[1], lw.z, lw.t, lw.rh, lw.part, S, lw.ctr, maxit);
+                        if (launch_pdl(bs_z_kernel, dim3(nb), dim3(LB), 0, st, N, fd, cd, lw.z, lw.invD, status, w1, lw.q[1], S)) return 1;
+                        if (launch_pdl(v4 ? bs_spmv_kernel<true> : bs_spmv_kernel<false>, dim3(nb), dim3(LB), 0, st, Af, N, lw.q[1], lw.t, nullptr, lw.z, lw.part, S, lw.ctr)) return 1;
+                        if (launch_pdl(bs_update_kernel, dim3(nb), dim3(LB), 0, st, N, lw.e, lw.r, lw.p[1], lw.q[1], lw.z, lw.t, lw.rh, lw.part, S, lw.ctr, maxit)) return 1;
                     }
                 }
                 CB_CHECK_LAUNCH();
@@ -2314,8 +2353,8 @@ int learned_train(LearnedWork& lw, const OpSym& A, const uint8_t* status, const 
             for (int l = 1; l < lw.nLev; ++l) {
                 Level& c = lw.lev[l];
                 const Level& f = lw.lev[l - 1];
-                restrict_kernel<<<restrict_grid(dims_of(c)), 256, 0, st>>>(dims_of(f), dims_of(c), l == 1 ? lw.r : f.u, nullptr, nullptr, 1.f,
-                                                                           c.u, c.w, c.gain, nullptr, nullptr, nullptr, 0.f, S);
+                if (launch_pdl(restrict_kernel, dim3(restrict_grid(dims_of(c))), dim3(256), 0, st, dims_of(f), dims_of(c), l == 1 ? lw.r : f.u, nullptr, nullptr, 1.f,
+                                                                           c.u, c.w, c.gain, nullptr, nullptr, nullptr, 0.f, S)) return 1;
                 if (l >= lw.netFrom && l <= lw.netTo) {
                     // y = (net(x) - net(-x)) / 2: the two evaluations get dL/dy / 2 and -dL/dy / 2
                     nets[nn] = &c.net; dys[nn] = c.w; scale[nn++] = 0.5f;
