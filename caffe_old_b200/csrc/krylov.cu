@@ -1025,10 +1025,12 @@ static int sm_count() {
     return g_numSM;
 }
 
-// Shape of a persistent launch over n work items (one per thread and step of the sweep): blocks
-// of 512 threads, as few as the items fill, since a reduction waits for every block (1.5 us on
-// 8 blocks, 2.4 on 148); past one block per SM the blocks grow to what the kernel's registers
-// allow and the sweep takes several steps.
+// Shape of a persistent launch over n work items (one per thread and step of the sweep): as many
+// threads per block, a power of two from 128, as give every item a thread of its own on all SMs, up to
+// what the kernel's registers allow; past that the sweep takes several steps.  Fewer, fuller blocks make
+// the reduction cheaper (1.5 us on 8 blocks, 2.4 on 148), but the loads of a sweep want every SM: CG
+// per iteration, us, blocks of 512 and up against this rule: 34x32x32 7.4 and 5.7, 44x40x38 7.9 and
+// 5.7, 56x50x48 8.0 and 6.4, 101x67x53 10.3 both.
 template <auto Kernel>
 static int launch_coop(long long n, void** params, cudaStream_t st) {
     static const int maxThreads = [] {
@@ -1037,7 +1039,7 @@ static int launch_coop(long long n, void** params, cudaStream_t st) {
     }();
     const int nsm = sm_count();
     int block = 128;
-    while (block < maxThreads && n > (long long)block * std::min(nsm, 32)) block = std::min(2 * block, maxThreads);
+    while (block < maxThreads && n > (long long)block * nsm) block = std::min(2 * block, maxThreads);
     const int grid = (int)std::min<long long>(nsm, (n + block - 1) / block);
     CB_CUDA(cudaLaunchCooperativeKernel((const void*)Kernel, dim3(grid), dim3(block), params, 0, st));
     return 0;
