@@ -142,128 +142,65 @@ __device__ __forceinline__ void project_mean(GridRed& grid, double* b, long long
 // are formed at the stencil neighbours from the stored vectors; P and V are double-buffered.
 // At a check (the recursive norm meets the tolerance, maxit, a breakdown) x takes the half-finished
 // iteration's update and the true residual decides, as in CG.
-// y = A f for W cells from c on; f.vec(e, o): values of W cells from e on, f.one(q, e): of one cell
-template <int NR, int W, class Op, class F>
-__device__ __forceinline__ void apply_w(const Op& A, long long c, F&& f, double (&y)[NR][W]) {
-    static_assert(W == 1, "only the symmetric operator has a group form");
-    double t[NR];
-    apply<NR>(A, c, [&](int q, long long e) { return f.one(q, e); }, t);
-#pragma unroll
-    for (int q = 0; q < NR; ++q) y[q][0] = t[q];
-}
-template <int NR, int W, class F>
-__device__ __forceinline__ void apply_w(const OpSym& A, long long c, F&& f, double (&y)[NR][W]) {
-    double o[W], n[W], s[W], t[W], b[W], kP[W], kE[W], kN[W], kS[W], kT[W], kB[W];
-    const uint2 gw = A.gh.n > 0 ? __ldg(A.gh.words + (c >> 5)) : make_uint2(0u, 0u);
-    f.vec(c, o);
-    f.vec(c + A.nI, n); f.vec(c - A.nI, s);
-    f.vec(c + A.nIJ, t); f.vec(c - A.nIJ, b);
-    const double w = f.one(0, c - 1), e = f.one(0, c + W), kw = A.aE[c - 1];
-    ldw<double, W>(A.aP + c, kP); ldw<double, W>(A.aE + c, kE);
-    ldw<double, W>(A.aN + c, kN); ldw<double, W>(A.aN + c - A.nI, kS);
-    ldw<double, W>(A.aT + c, kT); ldw<double, W>(A.aT + c - A.nIJ, kB);
-#pragma unroll
-    for (int m = 0; m < W; ++m)
-        y[0][m] = kP[m] * o[m] + kE[m] * (m + 1 < W ? o[m + 1 < W ? m + 1 : 0] : e) + (m ? kE[m ? m - 1 : 0] : kw) * (m ? o[m ? m - 1 : 0] : w)
-                  + kN[m] * n[m] + kS[m] * s[m] + kT[m] * t[m] + kB[m] * b[m];
-#pragma unroll
-    for (int m = 0; m < W; ++m)   // W divides 32: the group's cells share a word
-        if (is_ghost(gw, c + m)) {
-            double g[1];
-            ghost_row<1>(A.gh, ghost_index(gw, c + m), [&](int q, long long e_) { return f.one(q, e_); }, g);
-            y[0][m] = g[0];
-        }
+// y = A x of one row for the two sweeps.  What bounds a sweep at 40^3 to 100^3 is the chain of loads of
+// each step (2.5 us a step): a row's own values are loaded ahead of the product and the product's
+// operands before its first operation.  One cell per thread: pairs of cells halve the steps, but leave
+// half the loads in flight at the same registers and run the two cells' ghost rows one after the
+// other (us per iteration, FP64, sphere: 64x44x42 10.0 against 12.3, 80x52x50 12.9 against 14.7,
+// 96x64x64 16.8 against 21.1; 13.0 against 13.2 at 72x48x48 and, with the loads in the order of use, 10.3
+// against 13.5 at 75x39x41).  Ghost rows stay in the sweep: as items of their own after the stencil
+// rows they took 13.6 at 75x39x41 and 21.2 at 96x64x64.
+template <class Op, class X>
+__device__ __forceinline__ double row_product(const Op& A, long long c, X&& x) { double y[1]; apply<1>(A, c, x, y); return y[0]; }
+// every operand asked for before the first one is used
+template <class X>
+__device__ __forceinline__ double row_product(const OpSym& A, long long c, X&& x) {
+    const uint2 g = A.gh.n > 0 ? __ldg(A.gh.words + (c >> 5)) : make_uint2(0u, 0u);
+    const double o = x(0, c), n = x(0, c + A.nI), s = x(0, c - A.nI), t = x(0, c + A.nIJ), b = x(0, c - A.nIJ);
+    const double w = x(0, c - 1), e = x(0, c + 1), kW = A.aE[c - 1];
+    const double kP = A.aP[c], kE = A.aE[c], kN = A.aN[c], kS = A.aN[c - A.nI], kT = A.aT[c], kB = A.aT[c - A.nIJ];
+    double y = kP * o + kE * e + kW * w + kN * n + kS * s + kT * t + kB * b;
+    if (is_ghost(g, c)) { double v[1]; ghost_row<1>(A.gh, ghost_index(g, c), x, v); y = v[0]; }
+    return y;
 }
 
 struct BiVecs {
     double *x, *r, *s, *t, *rp;
     const double* invD;
-    long long N, PS;
+    long long N, t0, T;   // rows, this thread's first, and the step
 };
 
-// sweep 1:  x += xa P + xo S;  R = S - omega T;  P' = R + beta (P - omega V);  v = A P';  sums (rp, v)
-template <int NR, int W, class Op>
-__device__ __forceinline__ void bi_sweep1(const Op& A, const BiVecs& b, const double* P, const double* V, double* Pn, double* Vn, const bool (&run)[NR],
-                                          const double (&xa)[NR], const double (&xo)[NR], const double (&omega)[NR], const double (&beta)[NR],
-                                          double (&acc)[NR]) {
-    struct F {
-        const double *S, *Tt, *P, *V;
-        long long PS;
-        const double (&om)[NR], (&be)[NR];
-        __device__ __forceinline__ double one(int q, long long e) const {
-            const long long i = q * PS + e;
-            return (S[i] - om[q] * Tt[i]) + be[q] * (P[i] - om[q] * V[i]);
-        }
-        __device__ __forceinline__ void vec(long long e, double (&o)[W]) const {
-            double s[W], t[W], p[W], v[W];
-            ldw<double, W>(S + e, s); ldw<double, W>(Tt + e, t); ldw<double, W>(P + e, p); ldw<double, W>(V + e, v);
-#pragma unroll
-            for (int m = 0; m < W; ++m) o[m] = (s[m] - om[0] * t[m]) + be[0] * (p[m] - om[0] * v[m]);
-        }
-    } f{b.s, b.t, P, V, b.PS, omega, beta};
-    const long long step = W * (long long)gridDim.x * blockDim.x;
-    for (long long c = W * (blockIdx.x * (long long)blockDim.x + threadIdx.x); c < b.N; c += step) {
-        double y[NR][W], id[W];
-        apply_w<NR, W>(A, c, f, y);
-        ldw<double, W>(b.invD + c, id);
-#pragma unroll
-        for (int q = 0; q < NR; ++q) {
-            if (!run[q]) continue;
-            const long long i = q * b.PS + c;
-            double s[W], t[W], p[W], v[W], x[W], rp[W];
-            ldw<double, W>(b.s + i, s); ldw<double, W>(b.t + i, t); ldw<double, W>(P + i, p); ldw<double, W>(V + i, v);
-            ldw<double, W>(b.x + i, x); ldw<double, W>(b.rp + i, rp);
-#pragma unroll
-            for (int m = 0; m < W; ++m) {
-                x[m] = x[m] + (xa[q] * p[m] + xo[q] * s[m]);
-                s[m] = s[m] - omega[q] * t[m];
-                p[m] = s[m] + beta[q] * (p[m] - omega[q] * v[m]);
-                acc[q] += rp[m] * y[q][m];
-                v[m] = id[m] * y[q][m];
-            }
-            stw<double, W>(b.x + i, x); stw<double, W>(b.r + i, s); stw<double, W>(Pn + i, p); stw<double, W>(Vn + i, v);
-        }
+// sweep 1:  x += xa P + xo S;  R = S - omega T;  P' = R + beta (P - omega V);  v = A P';  sum (rp, v)
+template <class Op>
+__device__ __forceinline__ double bi_sweep1(const Op& A, const BiVecs& b, const double* P, const double* V, double* Pn, double* Vn,
+                                            double alpha, double omega, double beta) {
+    double acc = 0.;
+    auto next = [&](int, long long e) { return (b.s[e] - omega * b.t[e]) + beta * (P[e] - omega * V[e]); };
+    for (long long c = b.t0; c < b.N; c += b.T) {
+        const double id = b.invD[c], x = b.x[c], rp = b.rp[c];
+        const double y = row_product(A, c, next);
+        const double s = b.s[c], t = b.t[c], p = P[c], v = V[c];
+        const double r = s - omega * t;
+        b.x[c] = x + (alpha * p + omega * s);
+        b.r[c] = r;
+        Pn[c] = r + beta * (p - omega * v);
+        Vn[c] = id * y;
+        acc += rp * y;
     }
+    return acc;
 }
 
 // sweep 2:  S = R - alpha V;  t = A S;  sums (t, s), (t, t), (rp, s), (rp, t), (s, s)
-template <int NR, int W, class Op>
-__device__ __forceinline__ void bi_sweep2(const Op& A, const BiVecs& b, const double* V, const bool (&run)[NR], const double (&alpha)[NR],
-                                          double (&acc)[5 * NR]) {
-    struct F {
-        const double *R, *V;
-        long long PS;
-        const double (&al)[NR];
-        __device__ __forceinline__ double one(int q, long long e) const { return R[q * PS + e] - al[q] * V[q * PS + e]; }
-        __device__ __forceinline__ void vec(long long e, double (&o)[W]) const {
-            double r[W], v[W];
-            ldw<double, W>(R + e, r); ldw<double, W>(V + e, v);
-#pragma unroll
-            for (int m = 0; m < W; ++m) o[m] = r[m] - al[0] * v[m];
-        }
-    } f{b.r, V, b.PS, alpha};
-    const long long step = W * (long long)gridDim.x * blockDim.x;
-    for (long long c = W * (blockIdx.x * (long long)blockDim.x + threadIdx.x); c < b.N; c += step) {
-        double y[NR][W], id[W];
-        apply_w<NR, W>(A, c, f, y);
-        ldw<double, W>(b.invD + c, id);
-#pragma unroll
-        for (int q = 0; q < NR; ++q) {
-            if (!run[q]) continue;
-            const long long i = q * b.PS + c;
-            double s[W], v[W], rp[W];
-            ldw<double, W>(b.r + i, s); ldw<double, W>(V + i, v); ldw<double, W>(b.rp + i, rp);
-#pragma unroll
-            for (int m = 0; m < W; ++m) {
-                s[m] = s[m] - alpha[q] * v[m];
-                const double d = diag_of(A, c + m), sv = (d != 0. ? d : 1.) * s[m], tv = y[q][m];
-                acc[5 * q] += tv * sv; acc[5 * q + 1] += tv * tv;
-                acc[5 * q + 2] += rp[m] * sv; acc[5 * q + 3] += rp[m] * tv;
-                acc[5 * q + 4] += sv * sv;
-                v[m] = id[m] * y[q][m];
-            }
-            stw<double, W>(b.s + i, s); stw<double, W>(b.t + i, v);
-        }
+template <class Op>
+__device__ __forceinline__ void bi_sweep2(const Op& A, const BiVecs& b, const double* V, double alpha, double (&acc)[5]) {
+    auto next = [&](int, long long e) { return b.r[e] - alpha * V[e]; };
+    for (long long c = b.t0; c < b.N; c += b.T) {
+        const double id = b.invD[c], d = diag_of(A, c), rp = b.rp[c];
+        const double t = row_product(A, c, next);
+        const double S = b.r[c] - alpha * V[c], s = (d != 0. ? d : 1.) * S;
+        b.s[c] = S;
+        b.t[c] = id * t;
+        acc[0] += t * s; acc[1] += t * t; acc[2] += rp * s; acc[3] += rp * t; acc[4] += s * s;
     }
 }
 
@@ -276,129 +213,75 @@ __device__ __forceinline__ void bi_scalars(const double* t, double alpha, double
     rho = rn;
 }
 
-template <int NR, class Op, int W>
-__global__ void __launch_bounds__(W == 2 ? 640 : 512) bicgstab_kernel(Op A, KArgs a) {
+template <class Op>
+__global__ void __launch_bounds__(512) bicgstab_kernel(Op A, KArgs a) {
     if (a.skip_if_ok && *a.skip_if_ok == 0) return;   // uniform across the grid: no barrier is reached
     if (a.skip_if_ok && blockIdx.x == 0 && threadIdx.x == 0 && a.fallbacks) atomicAdd(a.fallbacks, 1);
     GridRed grid(a.partials);
-    const long long N = a.N, PS = a.PS;
+    const long long N = a.N;
     const long long T = (long long)gridDim.x * blockDim.x;
     const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const double* invD = a.invD;
-    if (NR == 1 && a.project) project_mean(grid, const_cast<double*>(a.b), N, t0, T);
+    if (a.project) project_mean(grid, const_cast<double*>(a.b), N, t0, T);
     // ---- initial state: x = 0, r = rp = b (S holds it for the first sweep, with P = V = T = 0)
-    double bb[NR];
+    double bb[1];
     {
-        double acc[NR];
-#pragma unroll
-        for (int q = 0; q < NR; ++q) acc[q] = 0.;
-        for (long long c = t0; c < N; c += T)
-#pragma unroll
-            for (int q = 0; q < NR; ++q) {
-                const double bv = a.b[q * PS + c];
-                a.x[q * PS + c] = 0.;
-                a.s[q * PS + c] = invD[c] * bv;
-                a.rp[q * PS + c] = bv;
-                a.t[q * PS + c] = 0.; a.p[0][q * PS + c] = 0.; a.v[0][q * PS + c] = 0.;
-                acc[q] += bv * bv;
-            }
-        grid.sum<NR>(acc, bb);
-    }
-    double rho[NR], alpha[NR], omega[NR], beta[NR], tol2[NR], relres[NR];
-    int it[NR], status[NR];
-    bool done[NR];
-#pragma unroll
-    for (int q = 0; q < NR; ++q) {
-        rho[q] = bb[q]; alpha[q] = 0.; omega[q] = 0.; beta[q] = 0.;
-        tol2[q] = fmax(a.rtol * a.rtol * bb[q], a.atol * a.atol);
-        it[q] = 0; relres[q] = 0.;
-        // x = 0 already meets the absolute floor: nothing to do (relative residual 1)
-        done[q] = !(bb[q] > 0.) || bb[q] <= tol2[q];
-        if (bb[q] > 0. && done[q]) relres[q] = 1.;
-        status[q] = bb[q] != bb[q] ? 3 : 0;
-    }
-    BiVecs v;
-    v.x = a.x; v.r = a.r; v.s = a.s; v.t = a.t; v.rp = a.rp; v.invD = invD; v.N = N; v.PS = PS;
-    int cur = 0;
-    while (true) {
-        bool run[NR], needT[NR], any = false;
-#pragma unroll
-        for (int q = 0; q < NR; ++q) { run[q] = !done[q]; any |= run[q]; needT[q] = false; }
-        if (!any) break;
-        // ---- sweep 1
-        {
-            double acc[NR], rv[NR];
-#pragma unroll
-            for (int q = 0; q < NR; ++q) acc[q] = 0.;
-            bi_sweep1<NR, W>(A, v, a.p[cur], a.v[cur], a.p[cur ^ 1], a.v[cur ^ 1], run, alpha, omega, omega, beta, acc);
-            grid.sum<NR>(acc, rv);
-#pragma unroll
-            for (int q = 0; q < NR; ++q) {
-                alpha[q] = omega[q] = 0.;   // x is up to date with R
-                if (!run[q]) continue;
-                if (rv[q] == 0. || rv[q] != rv[q]) { needT[q] = true; run[q] = false; }
-                else alpha[q] = rho[q] / rv[q];
-            }
-        }
-        cur ^= 1;
-        // ---- sweep 2
-        {
-            double acc[5 * NR], tot[5 * NR];
-#pragma unroll
-            for (int q = 0; q < 5 * NR; ++q) acc[q] = 0.;
-            bi_sweep2<NR, W>(A, v, a.v[cur], run, alpha, acc);
-            grid.sum<5 * NR>(acc, tot);
-            bool anyT = false;
-#pragma unroll
-            for (int q = 0; q < NR; ++q) {
-                if (run[q]) {
-                    double rr;
-                    it[q] += 1;
-                    bi_scalars(tot + 5 * q, alpha[q], omega[q], beta[q], rho[q], rr);
-                    if (rr <= tol2[q] || omega[q] == 0. || it[q] >= a.maxit || rr != rr) needT[q] = true;
-                }
-                anyT |= needT[q];
-            }
-            if (!anyT) continue;
-        }
-        // ---- true residual r = b - A x of the right-hand sides being checked
-        for (long long c = t0; c < N; c += T)
-#pragma unroll
-            for (int q = 0; q < NR; ++q) {
-                const long long i = q * PS + c;
-                if (needT[q]) a.x[i] = a.x[i] + (alpha[q] * a.p[cur][i] + omega[q] * a.s[i]);
-            }
-        grid.sync();
-        double acc[NR], rrT[NR];
-#pragma unroll
-        for (int q = 0; q < NR; ++q) acc[q] = 0.;
+        double acc[1] = {0.};
         for (long long c = t0; c < N; c += T) {
-            double y[NR];
-            apply<NR>(A, c, [&](int q, long long e) { return a.x[q * PS + e]; }, y);
-#pragma unroll
-            for (int q = 0; q < NR; ++q) {
-                if (!needT[q]) continue;
-                const long long i = q * PS + c;
-                const double rt = a.b[i] - y[q];
-                a.s[i] = invD[c] * rt; a.rp[i] = rt;
-                a.t[i] = 0.; a.p[cur][i] = 0.; a.v[cur][i] = 0.;
-                acc[q] += rt * rt;
-            }
+            const double bv = a.b[c];
+            a.x[c] = 0.;
+            a.s[c] = invD[c] * bv;
+            a.rp[c] = bv;
+            a.t[c] = 0.; a.p[0][c] = 0.; a.v[0][c] = 0.;
+            acc[0] += bv * bv;
         }
-        grid.sum<NR>(acc, rrT);
-#pragma unroll
-        for (int q = 0; q < NR; ++q) {
-            if (!needT[q]) continue;
-            relres[q] = sqrt(rrT[q] / bb[q]);
-            if (rrT[q] <= tol2[q]) { done[q] = true; status[q] = 0; }
-            else if (rrT[q] != rrT[q]) { done[q] = true; status[q] = 3; }
-            else if (it[q] >= a.maxit) { done[q] = true; status[q] = 1; }
-            else { rho[q] = rrT[q]; alpha[q] = omega[q] = beta[q] = 0.; }   // restart from the true residual
+        grid.sum<1>(acc, bb);
+    }
+    double rho = bb[0], alpha = 0., omega = 0., beta = 0., relres = 0.;
+    const double tol2 = fmax(a.rtol * a.rtol * bb[0], a.atol * a.atol);
+    int it = 0, status = bb[0] != bb[0] ? 3 : 0;
+    // x = 0 already meets the absolute floor: nothing to do (relative residual 1)
+    bool done = !(bb[0] > 0.) || bb[0] <= tol2;
+    if (bb[0] > 0. && done) relres = 1.;
+    BiVecs v;
+    v.x = a.x; v.r = a.r; v.s = a.s; v.t = a.t; v.rp = a.rp; v.invD = invD; v.N = N;
+    v.t0 = t0; v.T = T;
+    int cur = 0;
+    while (!done) {
+        double rv[1], acc1[1];
+        acc1[0] = bi_sweep1(A, v, a.p[cur], a.v[cur], a.p[cur ^ 1], a.v[cur ^ 1], alpha, omega, beta);
+        grid.sum<1>(acc1, rv);
+        alpha = omega = 0.;   // x is up to date with R
+        cur ^= 1;
+        if (rv[0] != 0. && rv[0] == rv[0]) {
+            alpha = rho / rv[0];
+            double acc[5] = {0., 0., 0., 0., 0.}, tot[5], rr;
+            bi_sweep2(A, v, a.v[cur], alpha, acc);
+            grid.sum<5>(acc, tot);
+            it += 1;
+            bi_scalars(tot, alpha, omega, beta, rho, rr);
+            if (!(rr <= tol2 || omega == 0. || it >= a.maxit || rr != rr)) continue;
         }
+        // ---- true residual r = b - A x
+        for (long long c = t0; c < N; c += T) a.x[c] = a.x[c] + (alpha * a.p[cur][c] + omega * a.s[c]);
+        grid.sync();
+        double acc[1] = {0.}, rrT[1];
+        for (long long c = t0; c < N; c += T) {
+            double y[1];
+            apply<1>(A, c, [&](int, long long e) { return a.x[e]; }, y);
+            const double rt = a.b[c] - y[0];
+            a.s[c] = invD[c] * rt; a.rp[c] = rt;
+            a.t[c] = 0.; a.p[cur][c] = 0.; a.v[cur][c] = 0.;
+            acc[0] += rt * rt;
+        }
+        grid.sum<1>(acc, rrT);
+        relres = sqrt(rrT[0] / bb[0]);
+        if (rrT[0] <= tol2) { done = true; status = 0; }
+        else if (rrT[0] != rrT[0]) { done = true; status = 3; }
+        else if (it >= a.maxit) { done = true; status = 1; }
+        else { rho = rrT[0]; alpha = omega = beta = 0.; }   // restart from the true residual
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        for (int q = 0; q < NR; ++q) { a.out->iters[q] = it[q]; a.out->relres[q] = relres[q]; a.out->status[q] = status[q]; }
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) { a.out->iters[0] = it; a.out->relres[0] = relres; a.out->status[0] = status; }
 }
 
 // ------------------------------------------------------------------ BiCGStab, three right-hand sides
@@ -1091,15 +974,6 @@ static int run_cg(const Op& A, const Lat& L, const KspWork& w, KArgs& a, cudaStr
     return launch_coop<cg1_kernel<Op>>(A, a, st);
 }
 
-// Groups of two cells where the rows are even.
-static int run_bicgstab(const OpSym& A, const Lat& L, KArgs& a, cudaStream_t st) {
-    auto al = [](const void* p) { return ((uintptr_t)p & 15u) == 0; };
-    const bool v2 = L.nI % 2 == 0 && al(a.r) && al(a.s) && al(a.rp) && al(a.p[0]) && al(a.p[1]) && al(a.v[0]) && al(a.v[1]) && al(a.t) &&
-                    al(a.invD) && al(a.x) && al(A.aP) && al(A.aE) && al(A.aN) && al(A.aT);
-    void* params[2] = {const_cast<OpSym*>(&A), &a};
-    return v2 ? launch_coop<bicgstab_kernel<1, OpSym, 2>>(L.N / 2, params, st) : launch_coop<bicgstab_kernel<1, OpSym, 1>>(L.N, params, st);
-}
-
 int ksp_bicgstab(const Op7& A, int nr, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit,
                  cudaStream_t st, double atol) {
     if (ksp_small_fits(L)) return ksp_small(A, false, nr, b, x, L, w, rtol, maxit, st, 0, atol);
@@ -1110,7 +984,7 @@ int ksp_bicgstab(const Op7& A, int nr, const double* b, double* x, const Lat& L,
         CB_CUDA(cudaLaunchCooperativeKernel((const void*)bicgstab3_kernel<3, Op7>, dim3(2 * sm_count()), dim3(KB), params, 0, st));
         return 0;
     }
-    return launch_coop<bicgstab_kernel<1, Op7, 1>>(A, a, st);
+    return launch_coop<bicgstab_kernel<Op7>>(A, a, st);
 }
 
 int ksp_bicgstab_sym(const OpSym& A, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit,
@@ -1119,7 +993,7 @@ int ksp_bicgstab_sym(const OpSym& A, const double* b, double* x, const Lat& L, c
     if (prepare(A, L, w, st)) return 1;
     KArgs a = make_args(L, w, b, x, rtol, maxit, atol);
     a.project = project;
-    return run_bicgstab(A, L, a, st);
+    return launch_coop<bicgstab_kernel<OpSym>>(A, a, st);
 }
 
 int ksp_cg(const OpSym& A, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit, cudaStream_t st,
@@ -1146,7 +1020,7 @@ int ksp_csr(const OpCSR& A, int method, long long n, const double* b, double* x,
     if (prepare(A, L, w, st)) return 1;
     KArgs a = make_args(L, w, b, x, rtol, maxit, atol);
     for (int q = 0; q < 3; ++q) a.cs[q] = nullptr;
-    return method == CAFFE_KSP_CG_JACOBI_INT ? launch_coop<cg1_kernel<OpCSR>>(A, a, st) : launch_coop<bicgstab_kernel<1, OpCSR, 1>>(A, a, st);
+    return method == CAFFE_KSP_CG_JACOBI_INT ? launch_coop<cg1_kernel<OpCSR>>(A, a, st) : launch_coop<bicgstab_kernel<OpCSR>>(A, a, st);
 }
 
 int ksp_mixed_sym(const OpSym& A, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit,
@@ -1176,7 +1050,7 @@ int ksp_fallback_sym(const OpSym& A, int method, const double* b, double* x, con
     a.fallbacks = fallbacks;
     if (method == CAFFE_KSP_CG_JACOBI_INT) return run_cg(A, L, w, a, st);
     if (prepare(A, L, w, st)) return 1;
-    return run_bicgstab(A, L, a, st);
+    return launch_coop<bicgstab_kernel<OpSym>>(A, a, st);
 }
 
 }  // namespace cb
