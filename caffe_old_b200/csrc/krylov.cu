@@ -261,7 +261,8 @@ __global__ void __launch_bounds__(512) bicgstab_kernel(Op A, KArgs a) {
             it += 1;
             bi_scalars(tot, alpha, omega, beta, rho, rr);
             if (!(rr <= tol2 || omega == 0. || it >= a.maxit || rr != rr)) continue;
-        }
+        } else
+            it += 1;   // a breakdown counts: from the same residual it repeats, and maxit must end it
         // ---- true residual r = b - A x
         for (long long c = t0; c < N; c += T) a.x[c] = a.x[c] + (alpha * a.p[cur][c] + omega * a.s[c]);
         grid.sync();
@@ -458,7 +459,7 @@ __global__ void __launch_bounds__(KB, 2) bicgstab3_kernel(Op A, KArgs a) {
 #pragma unroll
         for (int q = 0; q < NR; ++q) {
             if (!run[q]) continue;
-            if (rv[q] == 0. || rv[q] != rv[q]) { needT[q] = true; run[q] = false; }
+            if (rv[q] == 0. || rv[q] != rv[q]) { needT[q] = true; run[q] = false; it[q] += 1; }   // counted: a breakdown may repeat
             else alpha[q] = rho[q] / rv[q];
         }
         // ---- phase 2: s = r - alpha v;  t = A D^-1 s;  (t, s), (t, t)

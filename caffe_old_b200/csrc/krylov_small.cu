@@ -296,7 +296,8 @@ __global__ void __launch_bounds__(SB) small_bicgstab_kernel(Op op, SmallArgs a) 
             beta = (rn / rho) * (alpha / omega);
             rho = rn;
             check = rr <= f.tol2 || omega == 0. || f.it >= a.maxit || rr != rr;
-        }
+        } else
+            f.it += 1;   // a breakdown counts: from the same residual it repeats, and maxit must end it
         if (check) {
             double rr;
             f.check(r, a.maxit, rr);

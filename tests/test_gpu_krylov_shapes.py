@@ -74,3 +74,21 @@ def test_cg_on_a_matrix_that_is_not_symmetric_runs_the_general_form():
     x, _, rr, st = _lib.ksp7_solve(shape, coef, b, "cg_jacobi", RTOL, 5000)
     assert st == 0 and rr <= RTOL
     assert seven_point_residual(shape, coef, x, b) <= 1e-11
+
+
+@pytest.mark.parametrize("n", [2, 32768, 40000])
+@pytest.mark.parametrize("entry", ["ksp7", "csr"])
+def test_bicgstab_breakdown_from_the_first_residual_ends_at_maxit(entry, n):
+    """Pairs of cells with the matrix (0 1; -1 0) and b = 1: (r, A r) is zero exactly, from every restart."""
+    even = np.arange(n) % 2 == 0
+    b = np.ones(n)
+    if entry == "ksp7":
+        coef = np.zeros((7, n))
+        coef[1][even], coef[2][~even] = 1.0, -1.0
+        with pytest.raises(_lib.CaffeError):   # the call's answer to a solve that ends at maxit
+            _lib.ksp7_solve((n, 1, 1), coef, b, "bicgstab_jacobi", RTOL, 7)
+    else:
+        col = np.arange(n) + np.where(even, 1, -1)
+        x, its, rr, st = _lib.csr_solve(np.arange(n + 1), col, np.where(even, 1.0, -1.0), b, "bicgstab_jacobi", RTOL, 0.0, 7)
+        assert st == 2 and its == 7 and rr == 1.0
+        assert not x.any()
