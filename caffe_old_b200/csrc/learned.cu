@@ -1866,12 +1866,15 @@ void learned_free_host(LearnedWork& lw) {
 }
 
 namespace {
+// Basis planes a multiple of four floats apart: the smoother's kernels read and write them as float4,
+// and a lattice's own plane stride is odd where its cell count is.
+long long fg_stride(const Lat& L) { return (L.PS + 3) & ~3ll; }
 int fg_alloc(LearnedWork& lw, int m) {
     if (lw.fgCap >= m) return 0;
     if (lw.fgCap > 0) { set_error("FGMRES restart length cannot grow after the first FGMRES solve"); return 1; }
     const Lat& L = lw.L;
-    lw.fgV = static_cast<float*>(lw.alloc(sizeof(float) * (size_t)L.PS * (m + 1), lw.allocCtx));
-    lw.fgZ = static_cast<float*>(lw.alloc(sizeof(float) * (size_t)L.PS * m, lw.allocCtx));
+    lw.fgV = static_cast<float*>(lw.alloc(sizeof(float) * (size_t)fg_stride(L) * (m + 1), lw.allocCtx));
+    lw.fgZ = static_cast<float*>(lw.alloc(sizeof(float) * (size_t)fg_stride(L) * m, lw.allocCtx));
     lw.fgScal = lw.alloc(sizeof(FgScal), lw.allocCtx);
     lw.fgPart = static_cast<double*>(lw.alloc(sizeof(double) * (size_t)(FGM + 1) * FG_DOT_BLOCKS, lw.allocCtx));
     if (!lw.fgV || !lw.fgZ || !lw.fgScal || !lw.fgPart) { set_error("FGMRES workspace allocation failed"); return 1; }
@@ -1917,7 +1920,7 @@ int learned_solve(LearnedWork& lw, const OpSym& A, const uint8_t* status, const 
     const int m = lw.restart < 1 ? 1 : (lw.restart > FGM ? FGM : lw.restart);
     if (method == LEARN_INNER_FGMRES && fg_alloc(lw, m)) return 1;
     FgScal* F = static_cast<FgScal*>(lw.fgScal);
-    const long long PS = L.PS;
+    const long long PS = fg_stride(L);
     if (method != LEARN_INNER_FCG) {
         count_active_kernel<<<nb, LB, 0, st>>>(N, status, lw.part);
         count_finish<<<1, LB, 0, st>>>(lw.part, nb, lw.mean + 1);
