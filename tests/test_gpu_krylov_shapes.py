@@ -92,3 +92,25 @@ def test_bicgstab_breakdown_from_the_first_residual_ends_at_maxit(entry, n):
         x, its, rr, st = _lib.csr_solve(np.arange(n + 1), col, np.where(even, 1.0, -1.0), b, "bicgstab_jacobi", RTOL, 0.0, 7)
         assert st == 2 and its == 7 and rr == 1.0
         assert not x.any()
+
+
+@pytest.mark.parametrize("method", ["bicgstab_jacobi", "cg_jacobi"])
+@pytest.mark.parametrize("width", [1, 7, 8, 9, 21])
+@pytest.mark.parametrize("n", [21, 3001, 8000, 16384, 20011, 33000])
+def test_compressed_rows_shorter_and_longer_than_the_registers_hold(n, width, method):
+    """Rows of 1 to `width` entries that reach over the whole matrix, symmetric for CG; the bound is the
+    stopping test's, as above."""
+    rng = np.random.default_rng(n + width)
+    if method == "cg_jacobi":   # symmetric: pairs (i, n - 1 - i) and bands, each entry with its mirror image
+        offs = np.unique(np.concatenate([[0], *[[-o, o] for o in rng.integers(1, n, (width - 1) // 2)]]).astype(int))
+        rows = [np.unique(np.clip(i + offs, 0, n - 1)[(i + offs >= 0) & (i + offs < n)]) for i in range(n)]
+        vals = [np.where(c == i, 2.0 * width, -1.0) for i, c in enumerate(rows)]
+    else:
+        rows = [np.unique(np.append(rng.integers(0, n, rng.integers(0, width)), i)) for i in range(n)]
+        vals = [np.where(c == i, 2.0 * width, rng.uniform(-1.0, 1.0, c.size)) for i, c in enumerate(rows)]
+    ptr = np.concatenate([[0], np.cumsum([c.size for c in rows])])
+    col, val, b = np.concatenate(rows), np.concatenate(vals), rng.standard_normal(n)
+    x, _, rr, st = _lib.csr_solve(ptr, col, val, b, method, RTOL)
+    assert st == 0 and rr <= RTOL
+    ax = np.add.reduceat(val * x[col], ptr[:-1])
+    assert np.linalg.norm(b - ax) <= 1e-11 * np.linalg.norm(b)
