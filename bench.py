@@ -42,10 +42,11 @@ import numpy as np  # noqa: E402
 from caffe_old_b200 import cases as C  # noqa: E402
 
 HBM_FALLBACK = 6650.0
-# algorithmic bytes per matrix row and Krylov iteration of the dominant kernel
-# (fused Jacobi-PCG iteration: SpMV 72 + preconditioner 24 + x/r/p updates 64 + dot 8)
-PCG_BYTES_PER_ROW = 168.0
-BICGSTAB_BYTES_PER_ROW = 344.0
+# algorithmic bytes per matrix row and Krylov iteration of the dominant kernel: scaled CG, update
+# phase 64 (r, p, x read and written, q and the diagonal read) + product 40 (p, three planes, q written);
+# two-sweep BiCGStab, 15 planes in the first sweep and 10 in the second
+PCG_BYTES_PER_ROW = 104.0
+BICGSTAB_BYTES_PER_ROW = 200.0
 
 
 def peaks():
@@ -417,7 +418,7 @@ def run_b200(args, world, rank, local, pg):
             per_row = bytes_total / (N * p_iters) if p_iters > 0 else per_row
     else:
         per_row = PCG_BYTES_PER_ROW if method == "pcg" else BICGSTAB_BYTES_PER_ROW
-        kname = "cg1_kernel (persistent Jacobi-PCG, FP64)" if method == "pcg" else "bicgstab_kernel (persistent Jacobi-BiCGStab, FP64)"
+        kname = "cgs_kernel (persistent scaled Jacobi-CG, FP64)" if method == "pcg" else "bicgstab_kernel (persistent Jacobi-BiCGStab, FP64)"
     achieved = per_row * N * p_iters / (p_ms / 1e3) / 1e9 if (p_ms > 0 and per_row) else None
     # DRAM traffic from the ncu capture of the pyramid BiCGStab iteration; with the network stage
     # it describes the iterations after the hand-over, which are most of them

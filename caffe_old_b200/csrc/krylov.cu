@@ -7,22 +7,20 @@
 //   * BiCGStab (van der Vorst 1992), right-preconditioned, for the momentum system
 //     (three right-hand sides sharing one operator sweep) and for non-symmetric
 //     pressure-correction systems (immersed-boundary ghost rows);
-//   * CG (Hestenes-Stiefel; Chronopoulos-Gear single-reduction form), for the symmetric
-//     pressure-correction system.
+//   * CG (Hestenes-Stiefel 1952) with one reduction per iteration (Meurant 1987) on the
+//     symmetrically scaled system, for the symmetric pressure-correction system, and its
+//     Chronopoulos-Gear form where that scaling does not apply.
 // Every solve is one kernel launch: all blocks stay resident (cooperative launch) and
-// meet at grid barriers between the phases of an iteration; the dot products are summed
-// per block and then, in every block, over the block partials in a fixed order, so all
-// blocks take the same convergence decision and the result is bit-reproducible.  The
-// loop ends on the true residual ||b - A x|| <= rtol ||b|| (checked when the recursive
-// residual meets it; the iteration restarts from the true residual otherwise) or at
-// maxit, so no launch can run unbounded.
+// meet in grid reductions between the phases of an iteration (gridred.cuh); every block
+// sums the block partials in the same fixed order, so all blocks take the same
+// convergence decision and the result is bit-reproducible.  The loop ends on the true
+// residual ||b - A x|| <= rtol ||b|| (checked when the recursive residual meets it; the
+// iteration restarts from the true residual otherwise) or at maxit, so no launch can run
+// unbounded.  Systems of at most 32768 rows run inside one cluster (krylov_small.cu).
 //
 // Values written earlier in the same launch by other blocks are read with ordinary loads
-// after the grid barrier (whose device-scope fence orders them), never through the
-// read-only (non-coherent) path; only never-written inputs use __ldg.  Vectors that can be formed
-// from others are not stored: CG's search direction p = z + beta p_old and BiCGStab's
-// p = r + beta (p_old - omega v) and s = r - alpha v are recomputed at the stencil
-// neighbours instead of costing an extra pass and barrier.
+// after a reduction or barrier (whose release/acquire pair orders them), never through the
+// read-only (non-coherent) path; only never-written inputs use __ldg.
 #include <algorithm>
 #include <cstring>
 #include "cg_scaled.cuh"

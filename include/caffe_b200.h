@@ -27,7 +27,8 @@ enum caffe_solver_kind { CAFFE_SIMPLE = 0, CAFFE_PISO = 1, CAFFE_IBPISO = 2 };
  * the device implements BiCGStab and CG with Jacobi preconditioning. */
 enum caffe_ksp { CAFFE_KSP_BICGSTAB_SGS = 0, CAFFE_KSP_BICGSTAB_JACOBI = 1, CAFFE_KSP_CG_JACOBI = 2 };
 /* Form of the pressure-correction solve: plain FP64, FP32 inner solves inside FP64
- * iterative refinement, learned preconditioner, or both. */
+ * iterative refinement (symmetric systems of more than 32768 cells; others run FP64), learned
+ * preconditioner, or both. */
 enum caffe_p_form { CAFFE_P_FP64 = 0, CAFFE_P_MIXED = 1, CAFFE_P_LEARNED = 2, CAFFE_P_LEARNED_MIXED = 3 };
 
 /* Case parameters: the keys Simple / Piso / IbPiso read from case/case.info
