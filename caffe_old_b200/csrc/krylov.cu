@@ -752,8 +752,10 @@ __global__ void __launch_bounds__(1024) cgs_kernel(Op A, KArgs a) {
             alpha = beta = 0.;   // restart from the true residual, in the range of a singular A
             first = true;
             best = t[0];
-            if (a.project)
+            if (a.project) {
                 for (long long c = t0; c < N; c += T) v.r[c] = v.r[c] - sg * S[c] * (t[2] / (double)N);
+                grid.sync();     // the update deals the cells out in groups of W: r's next reader is another thread
+            }
         } else
             first = false;
     }
