@@ -26,6 +26,15 @@
 
 namespace cb {
 
+// A projected solve of a singular system restarts when (r, r) has grown by this factor from its smallest:
+// the round-off component of r along the null space never shrinks, and once the rest of r is down
+// to it alpha and beta drive r up without end; the restart projects it away.  On singular
+// 7-point systems (unit and lognormal conductances up to sigma 4, aspect ratios to 300) (r, r) rises by up
+// to 7e4 in a sound solve.  Other systems don't restart on growth: with a nearly singular matrix
+// (smallest eigenvalue 1e-9 of the diagonal) (r, r) rises further than this and then converges in 180 to 500
+// iterations, which restarting turned into 4000 without convergence.
+constexpr double CG_GROWTH = 1e6;
+
 template <class T, int W> struct VecOf;
 template <> struct VecOf<double, 1> { using type = double; };
 template <> struct VecOf<double, 2> { using type = double2; };

@@ -733,7 +733,7 @@ __global__ void __launch_bounds__(1024) cgs_kernel(Op A, KArgs a) {
         const bool broke = !cg_scalars(tot[0], tot[2], tot[3], alpha, beta);
         const bool stuck = broke && first;   // no direction from a fresh residual: a restart would not help
         if (tot[1] < best) best = tot[1];
-        if ((!first && (tot[1] <= tol2 || it >= a.maxit)) || !(tot[1] <= 1e6 * best) || broke) {
+        if ((!first && (tot[1] <= tol2 || it >= a.maxit)) || tot[1] != tot[1] || (a.project && tot[1] > CG_GROWTH * best) || broke) {
             // ---- true residual r = b - A x, x = S y
             double s[3] = {0., 0., 0.}, t[3];
             for (long long c = t0; c < N; c += T) {

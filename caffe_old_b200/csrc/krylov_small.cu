@@ -18,6 +18,7 @@
 #include <cooperative_groups.h>
 #include <cstring>
 
+#include "cg_scaled.cuh"
 #include "gridred.cuh"
 #include "krylov.cuh"
 #include "stencil.cuh"
@@ -376,7 +377,7 @@ __global__ void __launch_bounds__(SB) small_cg_kernel(Op op, SmallArgs a) {
         beta = next * d[0] > 0. ? next / d[0] : 0.;
         const bool broke = d[0] == 0. || d[2] == 0. || alpha != alpha || beta != beta, stuck = broke && first;
         if (d[1] < best) best = d[1];
-        if ((!first && (d[1] <= f.tol2 || f.it >= a.maxit)) || !(d[1] <= 1e6 * best) || broke) {
+        if ((!first && (d[1] <= f.tol2 || f.it >= a.maxit)) || d[1] != d[1] || (a.project && d[1] > CG_GROWTH * best) || broke) {
             double rr;
             f.check(r, a.maxit, rr);
             if (!f.done && stuck) { f.done = true; f.status = 2; }   // no direction from a fresh residual

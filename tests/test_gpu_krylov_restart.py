@@ -1,11 +1,13 @@
-"""Restarts of the pressure solve's Krylov kernels from the true residual, on systems above the 32768
-cells that one cluster holds."""
+"""When the Krylov kernels restart from the true residual, and when they must not: in one cluster (up
+to 32768 rows) and on the grid (above)."""
 import numpy as np
 import pytest
 
+from caffe_old_b200 import _lib
 from caffe_old_b200.solver import make_solver
 
 from helpers import small_cavity3d
+from test_zz_no_alloc import seven_point_residual, seven_point_system
 
 pytestmark = pytest.mark.gpu
 
@@ -33,3 +35,14 @@ def test_restarts_of_a_singular_system_repeat_bit_for_bit(n):
     for _ in range(5):
         again, st = pressure_solve(d, b)
         assert np.array_equal(again, first)
+
+
+@pytest.mark.parametrize("shape", [(20, 20, 20), (64, 64, 1), (31, 30, 29), (36, 32, 32), (33, 33, 33)])
+def test_cg_converges_on_a_nearly_singular_matrix(shape):
+    """Row sums of 1e-9: (r, r) rises far above its start before it falls, which is no reason to restart.
+    A solve takes a few hundred iterations; the residual is the stopping test's, evaluated on the host."""
+    coef, b = seven_point_system(shape, 21, True)
+    coef[0] = -coef[1:].sum(axis=0) - 1e-9
+    x, its, rr, st = _lib.ksp7_solve(shape, coef, b, "cg_jacobi", 1e-8, 2000)
+    assert st == 0 and rr <= 1e-8
+    assert seven_point_residual(shape, coef, x, b) <= 1.1e-8
