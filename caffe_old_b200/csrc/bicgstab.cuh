@@ -1,0 +1,24 @@
+// When the BiCGStab kernels that predict their scalars (krylov.cu, krylov_small.cu) have to restart.
+//
+// On convective systems (rp, r) falls to the round-off of its own terms long before r does, and the
+// iteration goes on with noise for rho.  That is harmless until rho comes out almost zero: the next
+// beta goes with 1 / rho and throws r up by orders of magnitude, for good.  Summed over the cells,
+// rho is a multiple of its terms' last place, such a rho is an exact zero, the next direction is
+// NaN and the solve restarts from the true residual; predicted as (rp, s) - omega (rp, t) it is an ordinary
+// small number.  So a rho below BI_FLOOR |rp| |r| restarts the process explicitly.
+//
+// Of 280 upwind convection-diffusion systems each on 64x64, 20x20x20 and 40x36x30 cells (Peclet numbers
+// to 1000, lognormal conductances) these reach 1e-9 within 4000 iterations: 255, 225 and 156
+// with rho summed over the cells, 176, 194 and 128 predicted without this rule, 266, 221 and 156 with it.  In 120
+// such systems on the CPU floors from 1e-18 to 1e-16 converge alike; from 1e-14 on restarts come too often.
+#pragma once
+#include "common.cuh"
+
+namespace cb {
+
+constexpr double BI_FLOOR = 3.4694469519536142e-18;   // 2^-58
+
+// rho = (rp, r), rp2 = (rp, rp), rr = (r, r)
+__device__ __forceinline__ bool bi_sound(double rho, double rp2, double rr) { return fabs(rho) > BI_FLOOR * sqrt(rp2 * fabs(rr)); }
+
+}  // namespace cb

@@ -23,6 +23,7 @@
 // read-only (non-coherent) path; only never-written inputs use __ldg.
 #include <algorithm>
 #include <cstring>
+#include "bicgstab.cuh"
 #include "cg_scaled.cuh"
 #include "gridred.cuh"
 #include "krylov.cuh"
@@ -202,13 +203,15 @@ __device__ __forceinline__ void bi_sweep2(const Op& A, const BiVecs& b, const do
     }
 }
 
-// omega, next beta and rho, and (r, r) from the sums of sweep 2
-__device__ __forceinline__ void bi_scalars(const double* t, double alpha, double& omega, double& beta, double& rho, double& rr) {
+// omega, next beta and rho, and (r, r) from the sums of sweep 2; true when the iteration may go on with
+// them (bi_sound)
+__device__ __forceinline__ bool bi_scalars(const double* t, double rp2, double alpha, double& omega, double& beta, double& rho, double& rr) {
     omega = t[1] == 0. ? 0. : t[0] / t[1];
     const double rn = t[2] - omega * t[3];
     rr = t[4] - 2. * omega * t[0] + omega * omega * t[1];
     beta = (rn / rho) * (alpha / omega);
     rho = rn;
+    return omega != 0. && rr == rr && bi_sound(rn, rp2, rr);
 }
 
 template <class Op>
@@ -235,7 +238,7 @@ __global__ void __launch_bounds__(512) bicgstab_kernel(Op A, KArgs a) {
         }
         grid.sum<1>(acc, bb);
     }
-    double rho = bb[0], alpha = 0., omega = 0., beta = 0., relres = 0.;
+    double rho = bb[0], rp2 = bb[0], alpha = 0., omega = 0., beta = 0., relres = 0.;
     const double tol2 = fmax(a.rtol * a.rtol * bb[0], a.atol * a.atol);
     int it = 0, status = bb[0] != bb[0] ? 3 : 0;
     // x = 0 already meets the absolute floor: nothing to do (relative residual 1)
@@ -257,8 +260,8 @@ __global__ void __launch_bounds__(512) bicgstab_kernel(Op A, KArgs a) {
             bi_sweep2(A, v, a.v[cur], alpha, acc);
             grid.sum<5>(acc, tot);
             it += 1;
-            bi_scalars(tot, alpha, omega, beta, rho, rr);
-            if (!(rr <= tol2 || omega == 0. || it >= a.maxit || rr != rr)) continue;
+            const bool sound = bi_scalars(tot, rp2, alpha, omega, beta, rho, rr);
+            if (sound && rr > tol2 && it < a.maxit) continue;
         } else
             it += 1;   // a breakdown counts: from the same residual it repeats, and maxit must end it
         // ---- true residual r = b - A x
@@ -278,7 +281,7 @@ __global__ void __launch_bounds__(512) bicgstab_kernel(Op A, KArgs a) {
         if (rrT[0] <= tol2) { done = true; status = 0; }
         else if (rrT[0] != rrT[0]) { done = true; status = 3; }
         else if (it >= a.maxit) { done = true; status = 1; }
-        else { rho = rrT[0]; alpha = omega = beta = 0.; }   // restart from the true residual
+        else { rho = rp2 = rrT[0]; alpha = omega = beta = 0.; }   // restart from the true residual
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) { a.out->iters[0] = it; a.out->relres[0] = relres; a.out->status[0] = status; }
 }

@@ -18,6 +18,7 @@
 #include <cooperative_groups.h>
 #include <cstring>
 
+#include "bicgstab.cuh"
 #include "cg_scaled.cuh"
 #include "gridred.cuh"
 #include "krylov.cuh"
@@ -299,7 +300,7 @@ __global__ void __launch_bounds__(SB) small_bicgstab_kernel(Op op, SmallArgs a) 
 #pragma unroll
     for (int k = 0; k < C; ++k) r[k] = p[k] = v[k] = t[k] = 0.;
     f.each([&](int k, int l) { r[k] = f.b[l]; });
-    double rho = f.bb, alpha = 0., omega = 0., beta = 0.;
+    double rho = f.bb, rp2 = f.bb, alpha = 0., omega = 0., beta = 0.;
     while (!f.done) {
         f.each([&](int k, int l) { p[k] = r[k] + beta * (p[k] - omega * v[k]); f.s.put(f.cl, l, f.id[l] * p[k]); });
         f.cl.sync();
@@ -328,7 +329,7 @@ __global__ void __launch_bounds__(SB) small_bicgstab_kernel(Op op, SmallArgs a) 
             const double rn = d[2] - omega * d[3], rr = d[4] - 2. * omega * d[0] + omega * omega * d[1];
             beta = (rn / rho) * (alpha / omega);
             rho = rn;
-            check = rr <= f.tol2 || omega == 0. || f.it >= a.maxit || rr != rr;
+            check = rr <= f.tol2 || omega == 0. || f.it >= a.maxit || rr != rr || !bi_sound(rn, rp2, rr);
         } else
             f.it += 1;   // a breakdown counts: from the same residual it repeats, and maxit must end it
         if (check) {
@@ -336,7 +337,7 @@ __global__ void __launch_bounds__(SB) small_bicgstab_kernel(Op op, SmallArgs a) 
             f.check(r, a.maxit, rr);
             // a restart from the true residual, if the solve goes on
             f.each([&](int k, int l) { f.rp[l] = r[k]; p[k] = v[k] = 0.; });
-            rho = rr; alpha = omega = beta = 0.;
+            rho = rp2 = rr; alpha = omega = beta = 0.;
         }
     }
     f.finish(a.out, rhs);

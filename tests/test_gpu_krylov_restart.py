@@ -46,3 +46,34 @@ def test_cg_converges_on_a_nearly_singular_matrix(shape):
     x, its, rr, st = _lib.ksp7_solve(shape, coef, b, "cg_jacobi", 1e-8, 2000)
     assert st == 0 and rr <= 1e-8
     assert seven_point_residual(shape, coef, x, b) <= 1.1e-8
+
+
+def convective_system(shape, seed, pe):
+    """Upwind convection in a rotating flow of cell Peclet number up to pe / 2, with a little reaction."""
+    nI, nJ, nK = shape
+    N = nI * nJ * nK
+    idx = np.arange(N)
+    i, j, k = idx % nI, (idx // nI) % nJ, idx // (nI * nJ)
+    u, v = pe * (j / nJ - 0.5), -pe * (i / nI - 0.5)     # through a cell's east and west, north and south faces
+    coef = np.zeros((7, N))
+    for q, (inside, into) in enumerate(((i < nI - 1, -u), (i > 0, u), (j < nJ - 1, -v), (j > 0, v), (k < nK - 1, 0 * u), (k > 0, 0 * u))):
+        coef[q + 1][inside] = (1.0 + np.maximum(into, 0.0))[inside]
+    coef[0] = -coef[1:].sum(axis=0) - 1e-3
+    return coef, np.random.default_rng(seed).standard_normal(N)
+
+
+@pytest.mark.parametrize("shape,peclets,most", [((64, 64, 1), (10.0, 30.0, 100.0, 300.0), 187_000), ((40, 36, 30), (10.0, 30.0), 112_000)])
+def test_bicgstab_restarts_on_an_almost_vanishing_rho(shape, peclets, most):
+    """Convective systems on which (rp, r) sinks to round-off.  How long one of them takes is chance; together,
+    with (rp, r) summed over the cells in every iteration, they take 124,500 and 75,000 iterations, and
+    the bound is half as many again (over 290,000 without the restarts, and some end at maxit).  The
+    residual is the stopping test's, evaluated on the host."""
+    total = 0
+    for pe in peclets:
+        for seed in range(12):
+            coef, b = convective_system(shape, seed, pe)
+            x, its, rr, st = _lib.ksp7_solve(shape, coef, b, "bicgstab_jacobi", 1e-9, 20000)
+            assert st == 0 and rr <= 1e-9
+            assert seven_point_residual(shape, coef, x, b) <= 1.1e-9
+            total += its
+    assert total <= most
