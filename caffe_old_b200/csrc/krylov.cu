@@ -997,14 +997,6 @@ int ksp_bicgstab_sym(const OpSym& A, const double* b, double* x, const Lat& L, c
     if (prepare(A, L, w, st)) return 1;
     KArgs a = make_args(L, w, b, x, rtol, maxit, atol);
     a.project = project;
-    // Above 4M rows the classic three-sweep order: the two-sweep form's predicted rho loses it there (two of
-    // four sphere lattices of 7.2 to 25.2M cells ended at maxit, all four converge in three sweeps);
-    // up to 3.1M cells both converge alike and two sweeps take 0.55 of the time.
-    if (L.N > (4ll << 20) && !project) {
-        void* params[2] = {const_cast<OpSym*>(&A), &a};
-        CB_CUDA(cudaLaunchCooperativeKernel((const void*)bicgstab3_kernel<1, OpSym>, dim3(2 * sm_count()), dim3(KB), params, 0, st));
-        return 0;
-    }
     return launch_coop<bicgstab_kernel<OpSym>>(A, a, st);
 }
 

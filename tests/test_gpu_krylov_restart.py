@@ -3,7 +3,8 @@ to 32768 rows) and on the grid (above)."""
 import numpy as np
 import pytest
 
-from caffe_old_b200 import _lib
+from caffe_old_b200 import _lib, precond as P
+from caffe_old_b200 import cases as C
 from caffe_old_b200.solver import make_solver
 
 from helpers import small_cavity3d
@@ -77,3 +78,16 @@ def test_bicgstab_restarts_on_an_almost_vanishing_rho(shape, peclets, most):
             assert seven_point_residual(shape, coef, x, b) <= 1.1e-9
             total += its
     assert total <= most
+
+
+def test_fp64_solve_behind_a_failed_learned_one_converges_on_a_large_lattice():
+    """Network parameters that are not numbers: every learned solve of the step fails at once, and the FP64
+    BiCGStab behind it solves the systems of a 6.3M-cell sphere, from rest."""
+    nodes, spec, _ = C.config5_sphere((240, 160, 164), p_form="learned_mixed")
+    d = make_solver(nodes, spec)
+    P.set_params(d, np.full_like(P.load_default(), np.nan))
+    P.set_mode(d, "network")
+    d.solve()
+    st = d.last_stats
+    assert st["fallbacks"] == st["p_solves"] > 0
+    assert st["p_res_max"] <= spec.p_rtol
