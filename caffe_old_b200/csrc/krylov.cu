@@ -254,7 +254,8 @@ __global__ void __launch_bounds__(512) bicgstab_kernel(Op A, KArgs a) {
         grid.sum<1>(acc1, rv);
         alpha = omega = 0.;   // x is up to date with R
         cur ^= 1;
-        if (rv[0] != 0. && rv[0] == rv[0]) {
+        const bool broke = rv[0] == 0. || rv[0] != rv[0];
+        if (!broke) {
             alpha = rho / rv[0];
             double acc[5] = {0., 0., 0., 0., 0.}, tot[5], rr;
             bi_sweep2(A, v, a.v[cur], alpha, acc);
@@ -262,11 +263,11 @@ __global__ void __launch_bounds__(512) bicgstab_kernel(Op A, KArgs a) {
             it += 1;
             const bool sound = bi_scalars(tot, rp2, alpha, omega, beta, rho, rr);
             if (sound && rr > tol2 && it < a.maxit) continue;
+            for (long long c = t0; c < N; c += T) a.x[c] = a.x[c] + (alpha * a.p[cur][c] + omega * a.s[c]);
+            grid.sync();
         } else
             it += 1;   // a breakdown counts: from the same residual it repeats, and maxit must end it
-        // ---- true residual r = b - A x
-        for (long long c = t0; c < N; c += T) a.x[c] = a.x[c] + (alpha * a.p[cur][c] + omega * a.s[c]);
-        grid.sync();
+        // ---- true residual r = b - A x.  After a breakdown x is what it was: P' may not be finite there
         double acc[1] = {0.}, rrT[1];
         for (long long c = t0; c < N; c += T) {
             double y[1];

@@ -91,3 +91,20 @@ def test_fp64_solve_behind_a_failed_learned_one_converges_on_a_large_lattice():
     st = d.last_stats
     assert st["fallbacks"] == st["p_solves"] > 0
     assert st["p_res_max"] <= spec.p_rtol
+
+
+@pytest.mark.parametrize("block,rhs", [([[-1, -1, 0], [2, 1, 0], [0, 2, -1]], [0, -1, -1]), ([[-1, -2, 0], [0, 1, -1], [0, 2, -1]], [-1, 1, 0])])
+@pytest.mark.parametrize("blocks", [3, 10000, 16384])
+def test_bicgstab_restarts_where_rho_is_exactly_zero(block, rhs, blocks):
+    """Blocks of three rows, all values small whole numbers or halves: after the first iteration x is finite, r is
+    not zero and (rp, r) is exactly zero in any order of summation; going on, the second beta is 0 / 0 and
+    the next direction not a number.  The solve restarts from the true residual with the x it has and takes a
+    few iterations more (condition numbers below 100)."""
+    block, rhs = np.array(block, dtype=float), np.array(rhs, dtype=float)
+    coef = np.zeros((7, 3 * blocks))
+    coef[0] = np.tile(np.diag(block), blocks)
+    coef[1] = np.tile([block[0, 1], block[1, 2], 0.0], blocks)
+    coef[2] = np.tile([0.0, block[1, 0], block[2, 1]], blocks)
+    x, _, rr, st = _lib.ksp7_solve((3 * blocks, 1, 1), coef, np.tile(rhs, blocks), "bicgstab_jacobi", 1e-12, 50)
+    assert st == 0 and rr <= 1e-12
+    assert np.linalg.norm(x.reshape(blocks, 3) - np.linalg.solve(block, rhs)) <= 1e-10 * np.linalg.norm(x)
