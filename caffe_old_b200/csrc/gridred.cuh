@@ -22,7 +22,10 @@ namespace cb {
 
 constexpr int GR_VALUES = 16;         // values of one reduction at most
 constexpr int GR_THREADS = 1024;      // threads of a block at most; one block per SM at most
-constexpr int GR_POLLS = 4000000;     // polls of the counter before a wait gives up (seconds)
+#ifndef CAFFE_GR_POLLS
+#define CAFFE_GR_POLLS 4000000
+#endif
+constexpr int GR_POLLS = CAFFE_GR_POLLS;   // polls of the counter before a wait gives up (4 million: seconds)
 
 // doubles of slot memory for a grid of `blocks` blocks: the counter's line, two buffers of partials
 inline size_t gr_doubles(int blocks) { return 16 + (size_t)2 * GR_VALUES * blocks; }
@@ -137,5 +140,89 @@ struct GridRed {
         return polls >= GR_POLLS;
     }
 };
+
+// The same sums with several blocks per SM and all partials added in block order (the three-sided
+// momentum solve): block partials, barrier, totals.
+constexpr int GR_ORDERED = 8;   // values of one such reduction at most
+// doubles for a grid of `blocks` blocks: the counter's line, two buffers of partials after it
+inline size_t gr_ordered_doubles(int blocks) { return 16 + (size_t)2 * GR_ORDERED * blocks; }
+__device__ __forceinline__ double ldcg(const double* p) { return *p; }   // coherent load after a grid barrier
+
+template <int K>
+__device__ __forceinline__ void gr_warp_sum(double (&v)[K]) {
+#pragma unroll
+    for (int q = 0; q < K; ++q)
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], off);
+}
+
+// block sums of v[0..K) into partials[blockIdx.x*GR_ORDERED + q]
+template <int K>
+__device__ void gr_block_partials(double (&v)[K], double* partials) {
+    __shared__ double sm[GR_ORDERED][32];
+    gr_warp_sum(v);
+    int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    if (lane == 0)
+#pragma unroll
+        for (int q = 0; q < K; ++q) sm[q][w] = v[q];
+    __syncthreads();
+    if (w == 0) {
+        double t[K];
+#pragma unroll
+        for (int q = 0; q < K; ++q) t[q] = lane < nw ? sm[q][lane] : 0.;
+        gr_warp_sum(t);
+        if (lane == 0)
+#pragma unroll
+            for (int q = 0; q < K; ++q) partials[blockIdx.x * GR_ORDERED + q] = t[q];
+    }
+    __syncthreads();
+}
+
+// sum of all blocks' partials, computed identically in every block
+template <int K>
+__device__ void gr_ordered_totals(const double* partials, double (&out)[K]) {
+    __shared__ double sm[GR_ORDERED][32];
+    double v[K];
+#pragma unroll
+    for (int q = 0; q < K; ++q) v[q] = 0.;
+    for (int g = threadIdx.x; g < (int)gridDim.x; g += blockDim.x)
+#pragma unroll
+        for (int q = 0; q < K; ++q) v[q] += ldcg(partials + (long long)g * GR_ORDERED + q);
+    gr_warp_sum(v);
+    int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    if (lane == 0)
+#pragma unroll
+        for (int q = 0; q < K; ++q) sm[q][w] = v[q];
+    __syncthreads();
+    if (w == 0) {
+        double t[K];
+#pragma unroll
+        for (int q = 0; q < K; ++q) t[q] = lane < nw ? sm[q][lane] : 0.;
+        gr_warp_sum(t);
+        __syncwarp();
+        if (lane == 0)
+#pragma unroll
+            for (int q = 0; q < K; ++q) sm[q][0] = t[q];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < K; ++q) out[q] = sm[q][0];
+    __syncthreads();
+}
+
+// Block partials, grid barrier, totals.  Partials alternate between two buffers: a block
+// that races ahead to the next reduction cannot overwrite a slot another block is still
+// summing, because it must first pass the barrier of the reduction in between.
+template <int K>
+__device__ __forceinline__ void gr_ordered_sum(GridRed& grid, double (&v)[K], double* partials, int& parity, double (&out)[K]) {
+    double* buf = partials + (long long)(parity & 1) * gridDim.x * GR_ORDERED;
+    gr_block_partials<K>(v, buf);
+    grid.sync();
+    gr_ordered_totals<K>(buf, out);
+    if (grid.dead)
+#pragma unroll
+        for (int q = 0; q < K; ++q) out[q] = __longlong_as_double(0x7ff8000000000000ll);
+    ++parity;
+}
 
 }  // namespace cb

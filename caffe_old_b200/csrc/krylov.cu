@@ -33,8 +33,6 @@
 
 namespace cb {
 
-__device__ __forceinline__ double ldcg(const double* p) { return *p; }   // coherent load after a grid barrier
-
 template <class Op>
 __global__ void inv_diag_kernel(Op A, long long N, double* invD, double* slots) {
     gr_clear(slots);
@@ -294,84 +292,10 @@ __global__ void __launch_bounds__(512) bicgstab_kernel(Op A, KArgs a) {
 // (0.36 against 0.38 ms per iteration at 128^3), and a solve is 3 to 15 iterations.  Two blocks of KB
 // threads per SM, partials summed in block order.
 constexpr int KB = 256;   // threads per block
-constexpr int KP = 8;     // partial slots per block
-
-template <int K>
-__device__ __forceinline__ void warp_sum(double (&v)[K]) {
-#pragma unroll
-    for (int q = 0; q < K; ++q)
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], off);
-}
-
-// block sums of v[0..K) into partials[blockIdx.x*KP + q]
-template <int K>
-__device__ void block_partials(double (&v)[K], double* partials) {
-    __shared__ double sm[KP][32];
-    warp_sum(v);
-    int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    if (lane == 0)
-#pragma unroll
-        for (int q = 0; q < K; ++q) sm[q][w] = v[q];
-    __syncthreads();
-    if (w == 0) {
-        double t[K];
-#pragma unroll
-        for (int q = 0; q < K; ++q) t[q] = lane < nw ? sm[q][lane] : 0.;
-        warp_sum(t);
-        if (lane == 0)
-#pragma unroll
-            for (int q = 0; q < K; ++q) partials[blockIdx.x * KP + q] = t[q];
-    }
-    __syncthreads();
-}
-
-// sum of all blocks' partials, computed identically in every block
-template <int K>
-__device__ void grid_totals(const double* partials, double (&out)[K]) {
-    __shared__ double sm[KP][32];
-    double v[K];
-#pragma unroll
-    for (int q = 0; q < K; ++q) v[q] = 0.;
-    for (int g = threadIdx.x; g < (int)gridDim.x; g += blockDim.x)
-#pragma unroll
-        for (int q = 0; q < K; ++q) v[q] += ldcg(partials + (long long)g * KP + q);
-    warp_sum(v);
-    int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    if (lane == 0)
-#pragma unroll
-        for (int q = 0; q < K; ++q) sm[q][w] = v[q];
-    __syncthreads();
-    if (w == 0) {
-        double t[K];
-#pragma unroll
-        for (int q = 0; q < K; ++q) t[q] = lane < nw ? sm[q][lane] : 0.;
-        warp_sum(t);
-        __syncwarp();
-        if (lane == 0)
-#pragma unroll
-            for (int q = 0; q < K; ++q) sm[q][0] = t[q];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < K; ++q) out[q] = sm[q][0];
-    __syncthreads();
-}
-
-// Block partials, grid barrier, totals.  Partials alternate between two buffers: a block
-// that races ahead to the next reduction cannot overwrite a slot another block is still
-// summing, because it must first pass the barrier of the reduction in between.
-template <int K>
-__device__ __forceinline__ void grid_reduce(GridRed& grid, double (&v)[K], double* partials, int& parity, double (&out)[K]) {
-    double* buf = partials + (long long)(parity & 1) * gridDim.x * KP;
-    block_partials<K>(v, buf);
-    grid.sync();
-    grid_totals<K>(buf, out);
-    ++parity;
-}
+constexpr int KB_PER_SM = 2;
 
 template <int NR, class Op>
-__global__ void __launch_bounds__(KB, 2) bicgstab3_kernel(Op A, KArgs a) {
+__global__ void __launch_bounds__(KB, KB_PER_SM) bicgstab3_kernel(Op A, KArgs a) {
     GridRed grid(a.partials);
     const long long N = a.N, PS = a.PS;
     const long long T = (long long)gridDim.x * blockDim.x;
@@ -398,7 +322,7 @@ __global__ void __launch_bounds__(KB, 2) bicgstab3_kernel(Op A, KArgs a) {
         double tmp[NR];
 #pragma unroll
         for (int q = 0; q < NR; ++q) tmp[q] = acc[q];
-        grid_reduce<NR>(grid, tmp, a.partials + 16, par, bb);
+        gr_ordered_sum<NR>(grid, tmp, a.partials + 16, par, bb);
     }
 
     double rho[NR], rho_old[NR], alpha[NR], omega[NR], tol2[NR];
@@ -456,7 +380,7 @@ __global__ void __launch_bounds__(KB, 2) bicgstab3_kernel(Op A, KArgs a) {
             double tmp[NR];
 #pragma unroll
             for (int q = 0; q < NR; ++q) tmp[q] = acc[q];
-            grid_reduce<NR>(grid, tmp, a.partials + 16, par, rv);
+            gr_ordered_sum<NR>(grid, tmp, a.partials + 16, par, rv);
         }
 #pragma unroll
         for (int q = 0; q < NR; ++q) {
@@ -486,7 +410,7 @@ __global__ void __launch_bounds__(KB, 2) bicgstab3_kernel(Op A, KArgs a) {
             double tmp[2 * NR];
 #pragma unroll
             for (int q = 0; q < 2 * NR; ++q) tmp[q] = acc[q];
-            grid_reduce<2 * NR>(grid, tmp, a.partials + 16, par, tot);
+            gr_ordered_sum<2 * NR>(grid, tmp, a.partials + 16, par, tot);
         }
 #pragma unroll
         for (int q = 0; q < NR; ++q) {
@@ -515,7 +439,7 @@ __global__ void __launch_bounds__(KB, 2) bicgstab3_kernel(Op A, KArgs a) {
             double tmp[2 * NR];
 #pragma unroll
             for (int q = 0; q < 2 * NR; ++q) tmp[q] = acc[q];
-            grid_reduce<2 * NR>(grid, tmp, a.partials + 16, par, tot);
+            gr_ordered_sum<2 * NR>(grid, tmp, a.partials + 16, par, tot);
         }
         bool anyT = false;
 #pragma unroll
@@ -551,7 +475,7 @@ __global__ void __launch_bounds__(KB, 2) bicgstab3_kernel(Op A, KArgs a) {
                 double tmp[NR];
 #pragma unroll
                 for (int q = 0; q < NR; ++q) tmp[q] = acc[q];
-                grid_reduce<NR>(grid, tmp, a.partials + 16, par, rrT);
+                gr_ordered_sum<NR>(grid, tmp, a.partials + 16, par, rrT);
             }
 #pragma unroll
             for (int q = 0; q < NR; ++q) {
@@ -938,7 +862,7 @@ static int launch_coop(const Op& op, KArgs& args, cudaStream_t st) {
     return launch_coop<Kernel>(args.N, params, st);
 }
 
-size_t krylov_partial_doubles() { return gr_doubles(sm_count()); }
+size_t krylov_partial_doubles() { return std::max(gr_doubles(sm_count()), gr_ordered_doubles(KB_PER_SM * sm_count())); }
 
 template <class Op>
 static int prepare(const Op& A, const Lat& L, const KspWork& w, cudaStream_t st) {
@@ -986,7 +910,7 @@ int ksp_bicgstab(const Op7& A, int nr, const double* b, double* x, const Lat& L,
     KArgs a = make_args(L, w, b, x, rtol, maxit, atol);
     if (nr == 3) {
         void* params[2] = {const_cast<Op7*>(&A), &a};
-        CB_CUDA(cudaLaunchCooperativeKernel((const void*)bicgstab3_kernel<3, Op7>, dim3(2 * sm_count()), dim3(KB), params, 0, st));
+        CB_CUDA(cudaLaunchCooperativeKernel((const void*)bicgstab3_kernel<3, Op7>, dim3(KB_PER_SM * sm_count()), dim3(KB), params, 0, st));
         return 0;
     }
     return launch_coop<bicgstab_kernel<Op7>>(A, a, st);

@@ -33,7 +33,7 @@ namespace cb {
 namespace {
 
 constexpr size_t SCRATCH_BYTES = size_t(16) << 20;
-// slots of the grid reductions: 128 bytes per SM, far below this;
+// slots of the grid reductions: 256 bytes per SM, far below this;
 // checked per call
 constexpr size_t PARTIAL_BYTES = size_t(128) << 10;
 constexpr int MAX_DEVICES = 64;
