@@ -17,6 +17,7 @@
 // values, so every face value is formed on the fly from the cell arrays.  Built with --fmad=false
 // and the operand order of the reference: everything outside the Krylov solve is bit for bit the
 // CPU restatement's.
+#include <algorithm>
 #include <climits>
 #include <cstring>
 #include <string>
@@ -65,6 +66,7 @@ struct caffe_coupled {
     double* x = nullptr;
     double* contMax = nullptr;
     KspWork kw = {};
+    int longest = 0;   // entries of the longest row
     int iters = 0, status = 0;
     double relres = 0.;
 
@@ -454,7 +456,7 @@ int launch_assemble(caffe_coupled* h, double dt, int part) {
 int launch_solve(caffe_coupled* h) {
     OpCSR A;
     A.ptr = h->ptr; A.col = h->col; A.val = h->val; A.diag = h->diag;
-    return ksp_csr(A, h->method, 4 * h->L.N, h->b, h->x, h->kw, h->rtol, h->maxit, h->st, h->atol);
+    return ksp_csr(A, h->method, 4 * h->L.N, h->longest, h->b, h->x, h->kw, h->rtol, h->maxit, h->st, h->atol);
 }
 
 int launch_post(caffe_coupled* h) {
@@ -539,6 +541,7 @@ int caffe_coupled_create(const double* nodes, int nNI, int nNJ, int nNK, const c
     if (cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking) != cudaSuccess) { set_error("stream creation failed"); return fail(); }
     std::vector<int> hptr, hcol, hdiag;
     build_structure(L, hptr, hcol, hdiag);
+    for (size_t r = 0; r + 1 < hptr.size(); ++r) h->longest = std::max(h->longest, hptr[r + 1] - hptr[r]);
     h->nnz = (long long)hcol.size();
     const long long nf[3] = {L.nFI, L.nFJ, L.nFK};
     const long long n4 = 4 * L.N;

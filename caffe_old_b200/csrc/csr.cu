@@ -2,6 +2,7 @@
 // reference's SparseMatrix does over PETSc's AIJ format (src/Math/SparseMatrix.cpp:49-106), handed
 // over once in compressed rows and solved by the persistent Jacobi-preconditioned Krylov kernels
 // (krylov.cu) on the device.  Used by the host layer's SparseMatrix / SparseVector classes.
+#include <algorithm>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -86,6 +87,8 @@ extern "C" int caffe_csr_solve(int n, const int* row_ptr, const int* col, const 
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev < 1) { set_error("no CUDA device available"); return 1; }
     const long long nnz = row_ptr[n];
+    int longest = 0;
+    for (int r = 0; r < n; ++r) longest = std::max(longest, row_ptr[r + 1] - row_ptr[r]);
     // one allocation for the matrix, the vectors and the solver's workspace (fifteen took a third of a
     // 6300-row solve)
     Arena d;
@@ -120,7 +123,7 @@ extern "C" int caffe_csr_solve(int n, const int* row_ptr, const int* col, const 
     CB_CHECK_LAUNCH();
     OpCSR A;
     A.ptr = dptr; A.col = dcol; A.val = dval; A.diag = ddiag;
-    if (ksp_csr(A, method, n, db, dx, w, rtol, maxit, st, atol)) return 1;
+    if (ksp_csr(A, method, n, longest, db, dx, w, rtol, maxit, st, atol)) return 1;
     KspOut o;
     CB_CUDA(cudaMemcpy(&o, w.out, sizeof(KspOut), cudaMemcpyDeviceToHost));
     CB_CUDA(cudaMemcpy(x, dx, sizeof(double) * n, cudaMemcpyDeviceToHost));

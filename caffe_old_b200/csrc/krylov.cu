@@ -940,12 +940,12 @@ int ksp_cg7(const Op7& A, const double* b, double* x, const Lat& L, const KspWor
     return run_cg(A, L, w, a, st);
 }
 
-int ksp_csr(const OpCSR& A, int method, long long n, const double* b, double* x, const KspWork& w, double rtol, int maxit,
+int ksp_csr(const OpCSR& A, int method, long long n, int longest, const double* b, double* x, const KspWork& w, double rtol, int maxit,
             cudaStream_t st, double atol) {
     Lat L;
     std::memset(&L, 0, sizeof(L));
     L.nI = (int)n; L.nJ = 1; L.nK = 1; L.N = n; L.nIJ = n; L.H = 0; L.PS = n;   // unpadded vectors
-    if (ksp_small_fits(L)) return ksp_small(A, method == CAFFE_KSP_CG_JACOBI_INT, b, x, L, w, rtol, maxit, st, atol);
+    if (ksp_small_fits_csr(n, longest)) return ksp_small(A, method == CAFFE_KSP_CG_JACOBI_INT, b, x, L, w, rtol, maxit, st, atol);
     if (prepare(A, L, w, st)) return 1;
     KArgs a = make_args(L, w, b, x, rtol, maxit, atol);
     for (int q = 0; q < 3; ++q) a.cs[q] = nullptr;

@@ -92,12 +92,14 @@ int ksp_mixed_sym(const OpSym& A, const double* b, double* x, const Lat& L, cons
 int ksp_fallback_sym(const OpSym& A, int method, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit,
                      cudaStream_t st, int project, const int* status, int* fallbacks, double atol = 0.);
 // Krylov solve of an n-row compressed-row system (vectors of n doubles, no halo): BiCGStab or CG
-// with Jacobi preconditioning, the same persistent kernels as the lattice solves.
-int ksp_csr(const OpCSR& A, int method, long long n, const double* b, double* x, const KspWork& w, double rtol, int maxit,
+// with Jacobi preconditioning, the same persistent kernels as the lattice solves; longest: entries of
+// the longest row.
+int ksp_csr(const OpCSR& A, int method, long long n, int longest, const double* b, double* x, const KspWork& w, double rtol, int maxit,
             cudaStream_t st, double atol = 0.);
 // The same solves inside one thread-block cluster, for systems whose vectors fit its registers and
 // shared memory (krylov_small.cu).  rhs right-hand sides PS apart, each solved by a cluster of its own.
 bool ksp_small_fits(const Lat& L);
+bool ksp_small_fits_csr(long long n, int longest);
 int ksp_small(const Op7& A, bool cgMethod, int rhs, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit,
               cudaStream_t st, int project, double atol);
 int ksp_small(const OpSym& A, bool cgMethod, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit, cudaStream_t st,

@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <cooperative_groups.h>
 #include <cstring>
+#include <type_traits>
 
 #include "bicgstab.cuh"
 #include "cg_scaled.cuh"
@@ -168,11 +169,11 @@ struct SmallOp {
 // Compressed rows: the first E entries of a thread's rows are kept in registers, each as its value and the
 // place of its column's cell in the cluster, so that a product is E independent shared-memory reads in
 // place of a chain through global memory (row bounds, then column, then the cell).  E = 8 covers the 5- and
-// 7-point rows, E = 5 is what fits beside four cells per thread; longer rows read the rest as before.  us per
-// BiCGStab iteration on 5-point rows: 6300 rows 6.7 -> 4.4, 12000 7.9 -> 5.9, 24000 19.6 -> 8.8.
+// 7-point rows; longer rows read the rest as before.  us per BiCGStab iteration on 5-point rows: 6300
+// rows 6.7 -> 4.4, 12000 7.9 -> 5.9.
 template <int C, int SB>
 struct SmallOp<OpCSR, C, SB> {
-    static constexpr int E = C <= 2 ? 8 : 5;
+    static constexpr int E = 8;
     OpCSR A;
     int p0[C], p1[C];
     double val[C][E];
@@ -474,7 +475,9 @@ int run(const Op& A, bool cgMethod, int rhs, const double* b, double* x, const L
     if (cells <= 256) { SMALL_LAUNCH(1, 256); }
     if (cells <= 512) { SMALL_LAUNCH(1, 512); }
     if (cells <= 1024) { SMALL_LAUNCH(2, 512); }
-    SMALL_LAUNCH(4, 512);
+    if constexpr (!std::is_same<Op, OpCSR>::value) { SMALL_LAUNCH(4, 512); }   // compressed rows: ksp_small_fits_csr
+    set_error("small-system solve: too many rows");
+    return 1;
 #undef SMALL_LAUNCH
 }
 
@@ -482,6 +485,16 @@ int run(const Op& A, bool cgMethod, int rhs, const double* b, double* x, const L
 
 bool ksp_small_fits(const Lat& L) {
     return L.N <= (long long)S_BLOCKS * S_THREADS * S_CELLS && small_bytes(7, shift_of(L.N), halo_of(L)) <= (size_t)S_BYTES && cluster_fits();
+}
+
+// Compressed rows: what lies beyond the registers is read entry by entry on 16 SMs, where the whole grid
+// has nine times as many, so long rows and many rows per thread belong there.  us per BiCGStab
+// iteration, cluster and grid, rows of 5 / 9 / 11 / 14 / 19 entries: 6000 rows 4.9 7.6 / 5.9 8.3 / 7.2 8.6 / 8.6 9.2 /
+// 12.9 10.5; 12000 rows 6.9 8.0 / 8.6 8.7 / 11.1 8.9 / 13.1 10.1 / 21.8 10.7; 26000 rows, four per thread, 11.4
+// 8.4 / 22.2 9.5 / 30.5 10.0 / 30.5 11.1 / 50.4 13.1.
+bool ksp_small_fits_csr(long long n, int longest) {
+    const bool one = n <= S_BLOCKS * S_THREADS, two = n <= 2 * S_BLOCKS * S_THREADS;   // rows per thread
+    return ((one && longest <= 14) || (two && longest <= 9)) && cluster_fits();
 }
 
 int ksp_small(const Op7& A, bool cgMethod, int rhs, const double* b, double* x, const Lat& L, const KspWork& w, double rtol, int maxit,
