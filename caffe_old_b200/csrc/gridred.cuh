@@ -178,9 +178,9 @@ __device__ void gr_block_partials(double (&v)[K], double* partials) {
     __syncthreads();
 }
 
-// sum of all blocks' partials, computed identically in every block
+// sum of all blocks' partials, computed identically in every block; NaN after a lost wait
 template <int K>
-__device__ void gr_ordered_totals(const double* partials, double (&out)[K]) {
+__device__ void gr_ordered_totals(const double* partials, bool lost, double (&out)[K]) {
     __shared__ double sm[GR_ORDERED][32];
     double v[K];
 #pragma unroll
@@ -202,7 +202,7 @@ __device__ void gr_ordered_totals(const double* partials, double (&out)[K]) {
         __syncwarp();
         if (lane == 0)
 #pragma unroll
-            for (int q = 0; q < K; ++q) sm[q][0] = t[q];
+            for (int q = 0; q < K; ++q) sm[q][0] = lost ? __longlong_as_double(0x7ff8000000000000ll) : t[q];
     }
     __syncthreads();
 #pragma unroll
@@ -218,10 +218,7 @@ __device__ __forceinline__ void gr_ordered_sum(GridRed& grid, double (&v)[K], do
     double* buf = partials + (long long)(parity & 1) * gridDim.x * GR_ORDERED;
     gr_block_partials<K>(v, buf);
     grid.sync();
-    gr_ordered_totals<K>(buf, out);
-    if (grid.dead)
-#pragma unroll
-        for (int q = 0; q < K; ++q) out[q] = __longlong_as_double(0x7ff8000000000000ll);
+    gr_ordered_totals<K>(buf, grid.dead, out);
     ++parity;
 }
 
