@@ -235,7 +235,7 @@ struct Frame {
         A.load(cl, op, mem + (S_VECS << a.shift), s, id);
         b = a.b + rhs * a.PS + s.base; xOut = a.x + rhs * a.PS + s.base;
         __syncthreads();
-        each([&](int, int l) { x[l] = 0.; rp[l] = b[l]; });
+        each([&](int, int l) { x[l] = 0.; });
         cl.sync();   // every block runs before its shared memory is written from outside
         double t[1];
         if (a.project)   // twice: see project_mean in krylov.cu
@@ -247,7 +247,7 @@ struct Frame {
                 each([&](int, int l) { b[l] = b[l] - mean; });
             }
         double v[1] = {0.};
-        each([&](int, int l) { v[0] += b[l] * b[l]; });
+        each([&](int, int l) { rp[l] = b[l]; v[0] += b[l] * b[l]; });
         sum(cl, v, t);
         bb = t[0];
         tol2 = fmax(a.rtol * a.rtol * bb, a.atol * a.atol);
