@@ -40,6 +40,7 @@
 
 #include "common.cuh"
 #include "cnn.cuh"
+#include "perdevice.h"
 
 namespace cb {
 
@@ -594,21 +595,13 @@ __global__ void __launch_bounds__(256) weight_grad_sum_kernel(const float* __res
     }
 }
 
-static long long weight_grad_ctas() {
-    int dev = 0, nsm = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    return 4LL * nsm;
-}
+static long long weight_grad_ctas() { return 4LL * sm_count(); }
 size_t weight_grad_part_floats() { return (size_t)weight_grad_ctas() * (WG_W + 32); }
 
 int launch_weight_grad_group(const WgSpec* specs, int n, float* grad, float* part, int* err, cudaStream_t st) {
     const size_t smem = 1024 + 2 * (size_t)WG_STAGE_BYTES;
-    static bool attr = false;
-    if (!attr) {
-        CB_CUDA(cudaFuncSetAttribute(weight_grad_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr = true;
-    }
+    static PerDevice<cudaError_t> attr;
+    CB_CUDA(attr.get(current_device(), [&] { return cudaFuncSetAttribute(weight_grad_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }));
     const long long most = weight_grad_ctas();
     double* dbPart = reinterpret_cast<double*>(part + (size_t)most * WG_W);
     for (int b = 0; b < n; b += CONV_MAX_JOBS) {
@@ -683,13 +676,13 @@ const CUtensorMap* cached_map(const __nv_bfloat16* in, const Lat& L) {
 int launch_conv3d_group(int epi, const ConvSpec* specs, int n, const __nv_bfloat16* wpack, const float* bias, int* err, cudaStream_t st,
                         const int* skip) {
     const size_t smem = conv_smem_bytes();
-    static bool attr = false;
-    if (!attr) {
-        CB_CUDA(cudaFuncSetAttribute(conv3d_tc_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        CB_CUDA(cudaFuncSetAttribute(conv3d_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        CB_CUDA(cudaFuncSetAttribute(conv3d_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr = true;
-    }
+    static PerDevice<cudaError_t> attr;
+    CB_CUDA(attr.get(current_device(), [&] {
+        cudaError_t e = cudaSuccess;
+        for (auto kernel : {conv3d_tc_kernel<0>, conv3d_tc_kernel<1>, conv3d_tc_kernel<2>})
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        return e;
+    }));
     for (int b = 0; b < n; b += CONV_MAX_JOBS) {
         ConvGroup g;
         std::memset(&g, 0, sizeof(g));

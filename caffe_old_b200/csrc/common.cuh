@@ -111,4 +111,11 @@ __device__ __forceinline__ double dot3(d3 a, d3 b) { return a.x * b.x + a.y * b.
 
 static inline int grid_for(long long n, int block) { return (int)((n + block - 1) / block); }
 
+static inline int current_device() {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return dev;
+}
+int sm_count();   // SMs of the current device
+
 }  // namespace cb

@@ -27,6 +27,7 @@
 #include "cg_scaled.cuh"
 #include "gridred.cuh"
 #include "krylov.cuh"
+#include "perdevice.h"
 #include "stencil.cuh"
 
 #define CAFFE_KSP_CG_JACOBI_INT 2   // caffe_ksp value of Jacobi-CG (include/caffe_b200.h)
@@ -826,15 +827,13 @@ __global__ void __launch_bounds__(1024) mixed_cg_kernel(OpSym A, MxArgs a) {
 }
 
 // ------------------------------------------------------------------ host side
-static int g_numSM = 0;
-
-static int sm_count() {
-    if (g_numSM == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&g_numSM, cudaDevAttrMultiProcessorCount, dev);
-    }
-    return g_numSM;
+int sm_count() {
+    static PerDevice<int> count;
+    const int dev = current_device();
+    return count.get(dev, [&] {
+        int n = 0;
+        return cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0 ? n : 148;
+    });
 }
 
 // Shape of a persistent launch over n work items (one per thread and step of the sweep): as many

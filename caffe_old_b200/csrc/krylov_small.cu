@@ -23,6 +23,7 @@
 #include "cg_scaled.cuh"
 #include "gridred.cuh"
 #include "krylov.cuh"
+#include "perdevice.h"
 #include "stencil.cuh"
 
 namespace cg = cooperative_groups;
@@ -403,11 +404,11 @@ size_t small_bytes(int planes, int shift, long long halo) { return sizeof(double
 template <auto Kernel, int SB>
 int launch_small(const void* op, SmallArgs& a, int rhs, int planes, int blocks, cudaStream_t st) {
     const size_t smem = small_bytes(planes, a.shift, a.halo);
-    static const bool ready = [] {
-        return cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S_BYTES) == cudaSuccess &&
-               cudaFuncSetAttribute(Kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-    }();
-    if (!ready) { set_error("small-system solve: kernel attributes refused"); return 1; }
+    static PerDevice<bool> ready;
+    if (!ready.get(current_device(), [] {
+            return cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S_BYTES) == cudaSuccess &&
+                   cudaFuncSetAttribute(Kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+        })) { set_error("small-system solve: kernel attributes refused"); return 1; }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks, rhs);
     cfg.blockDim = dim3(SB);
@@ -423,9 +424,10 @@ int launch_small(const void* op, SmallArgs& a, int rhs, int planes, int blocks, 
     return 0;
 }
 
-// whether the device runs a cluster of S_BLOCKS blocks of the largest form (asked once)
+// whether the current device runs a cluster of S_BLOCKS blocks of the largest form (asked once)
 bool cluster_fits() {
-    static const bool fits = [] {
+    static PerDevice<bool> fits;
+    return fits.get(current_device(), [] {
         auto k = small_bicgstab_kernel<Op7, S_CELLS, S_THREADS>;
         if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, S_BYTES) != cudaSuccess ||
             cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
@@ -444,8 +446,7 @@ bool cluster_fits() {
         int n = 0;
         if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) { cudaGetLastError(); return false; }
         return n >= 1;
-    }();
-    return fits;
+    });
 }
 
 // the fewest cells a block can hold with the whole cluster at work; at least a warp's

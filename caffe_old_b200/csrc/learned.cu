@@ -65,6 +65,7 @@
 #include "krylov.cuh"
 #include "learned.cuh"
 #include "stencil.cuh"
+#include "perdevice.h"
 
 namespace cb {
 
@@ -664,18 +665,13 @@ int launch_restrict_tma(const Dims3& fd, const Dims3& cd, const float* fin, cons
     if (md) maps.invD = *md;
     if (ms) maps.st = *ms;
     const size_t smemFull = 1024 + 2 * (size_t)RT_STAGE_BYTES, smemPre = 1024 + 3 * (size_t)RT_F_BYTES;
-    static bool attr = false;
-    static int nsm = 0;
-    if (!attr) {
-        CB_CUDA(cudaFuncSetAttribute(restrict_tma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemFull));
-        CB_CUDA(cudaFuncSetAttribute(restrict_tma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemPre));
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        attr = true;
-    }
+    static PerDevice<cudaError_t> attr;
+    CB_CUDA(attr.get(current_device(), [&] {
+        const cudaError_t e = cudaFuncSetAttribute(restrict_tma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemFull);
+        return e != cudaSuccess ? e : cudaFuncSetAttribute(restrict_tma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemPre);
+    }));
     const long long T = (long long)((cd.n0 + RCI - 1) / RCI) * ((cd.n1 + RCJ - 1) / RCJ) * ((cd.n2 + RCK - 1) / RCK);
-    const int sms = nsm > 0 ? nsm : 148;
+    const int sms = sm_count();
     if (pre) {
         const int grid = (int)std::min<long long>(T, 2LL * sms);   // two CTAs per SM
         if (launch_pdl(restrict_tma_kernel<true>, dim3(grid), dim3(RT_THREADS), smemPre, stream, maps, fd, cd, 0, scale, out, err, S)) return 1;
@@ -1760,8 +1756,8 @@ int apply_levels(LearnedWork& lw, const float* rfine, const uint8_t* status, int
             // the last level dealt out is held as well
             if (c.N > TAIL_OWN || q == 0) held = c.N;
         }
-        static const cudaError_t attr = cudaFuncSetAttribute(coarse_tail_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        CB_CUDA(attr);
+        static PerDevice<cudaError_t> attr;
+        CB_CUDA(attr.get(current_device(), [] { return cudaFuncSetAttribute(coarse_tail_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1); }));
         if (launch_pdl(coarse_tail_kernel, dim3(TAIL_BLOCKS), dim3(TAIL_THREADS), sizeof(float) * (size_t)(cells + 2 * held), st, ta, S)) return 1;
         CB_CHECK_LAUNCH();
     }

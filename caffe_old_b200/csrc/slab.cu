@@ -204,20 +204,10 @@ int run_phase(const Op& A, const SlabKsp& k, const SlabScal& s, cudaStream_t st,
     return K;
 }
 
-int sm_count_cached() {
-    static int n = 0;
-    if (n == 0) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
-            n = 148;
-    }
-    return n;
-}
-
 template <int NR, class Op>
 int dispatch(const Op& A, int phase, const SlabKsp& k, const SlabScal& s, cudaStream_t st) {
     if (k.o0 < 0 || k.o1 > k.L.N || k.o0 >= k.o1) { set_error("slab: empty or out-of-range owned cells"); return -1; }
-    const int sm = sm_count_cached();
+    const int sm = sm_count();
     switch (phase) {
         case SB_INIT: return run_phase<NR, Op, SB_INIT>(A, k, s, st, sm);
         case SB_P: return run_phase<NR, Op, SB_P>(A, k, s, st, sm);
