@@ -201,6 +201,13 @@ struct caffe_dev {
         return b ? b + L.H : nullptr;
     }
     static void* alloc_cb(size_t bytes, void* ctx) { return static_cast<caffe_dev*>(ctx)->dalloc<char>(bytes); }
+    int ensure_mixed() {
+        if (kw.fB[2]) return 0;
+        bool ok = true;
+        for (float** f : {&kw.fr, &kw.fq, &kw.fp, &kw.fe, &kw.fd, &kw.fB[0], &kw.fB[1], &kw.fB[2]}) ok = ok && (*f = fcell());
+        if (!ok) { set_error("device allocation failed (mixed-precision workspace)"); return 1; }
+        return 0;
+    }
     int ensure_learned() {
         if (haveLearned) return 0;
         if (learned_alloc(lw, L, &caffe_dev::alloc_cb, this)) return 1;
@@ -420,6 +427,7 @@ int ph_solve_pcorr(caffe_dev* h) {
         // the plain FP64 solve re-runs on the device when the refinement does not reach the
         // tolerance.  Systems with ghost rows take the FP64 BiCGStab below (krylov.cu), and those that one
         // cluster holds the FP64 solve there, where an iteration moves nothing and FP32 saves nothing
+        if (h->ensure_mixed()) return 1;
         rc = ksp_mixed_sym(A, h->pb, h->pc, h->L, h->kw, h->cs.p_rtol, h->cs.maxit, h->st, project, h->cs.p_atol);
         if (!rc) rc = ksp_fallback_sym(A, method, h->pb, h->pc, h->L, h->kw, h->cs.p_rtol, h->cs.maxit, h->st, 0,
                                        &h->kw.out->status[0], &h->acc->fallbacks, h->cs.p_atol);
@@ -675,13 +683,9 @@ int caffe_dev_create(const double* nodes, int nNI, int nNJ, int nNK, const caffe
     h->kw.t = h->cell(3); h->kw.invD = h->cell(1);
     // CG does not use the three planes of rp: they hold its scaled operator
     for (int q = 0; q < 3; ++q) h->kw.cs[q] = h->kw.rp ? h->kw.rp + q * L.PS : nullptr;
-    if (cs->p_form == CAFFE_P_MIXED) {
-        h->kw.fr = h->fcell(); h->kw.fq = h->fcell(); h->kw.fp = h->fcell(); h->kw.fe = h->fcell(); h->kw.fd = h->fcell();
-        for (int q = 0; q < 3; ++q) h->kw.fB[q] = h->fcell();
-        bool ok = h->kw.fr && h->kw.fq && h->kw.fp && h->kw.fe && h->kw.fd;
-        for (int q = 0; q < 3; ++q) ok = ok && h->kw.fB[q];
-        if (!ok) { set_error("device allocation failed (mixed-precision workspace)"); return fail(); }
-    }
+    // the FP32 planes where the mixed form runs FP32 (ph_solve_pcorr); a sphere that has no ghost rows is
+    // known only once it is placed
+    if (cs->p_form == CAFFE_P_MIXED && !h->ib && !ksp_small_fits(L) && h->ensure_mixed()) return fail();
     h->kw.partials = h->dalloc<double>(krylov_partial_doubles());
     h->kw.out = h->dalloc<KspOut>(1);
     h->chunkMax = h->dalloc<double>((size_t)(L.N / 1024 + 2));
