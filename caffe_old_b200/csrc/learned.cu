@@ -795,6 +795,7 @@ constexpr int TAIL_MAX_IN = 65536;      // cells of level lt-1
 constexpr int TAIL_OWN = 256;           // cells of a level that every block works out for itself
 constexpr int TAIL_PAIR = 8192;         // cells of the level above: order of the first pair (see above)
 constexpr int TAIL_THREADS = 1024, TAIL_BLOCKS = 16;
+constexpr int TAIL_BYTES = 2 * (TAIL_MAX + 2 * TAIL_OWN) * (int)sizeof(float);   // shared memory at most: one level dealt out and those below
 struct TailArgs {
     int n;                              // tail levels lt .. lt+n-1
     Dims3 d[LEARN_MAX_LEVELS + 1];      // d[0]: level lt-1; d[1..n]: the tail levels
@@ -1757,7 +1758,12 @@ int apply_levels(LearnedWork& lw, const float* rfine, const uint8_t* status, int
             if (c.N > TAIL_OWN || q == 0) held = c.N;
         }
         static PerDevice<cudaError_t> attr;
-        CB_CUDA(attr.get(current_device(), [] { return cudaFuncSetAttribute(coarse_tail_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1); }));
+        // u and w of the held levels: 20 KB where the pyramid goes down to 64 cells, up to 66 KB where it ends sooner
+        // (twelve levels of a line of more than 12 million cells)
+        CB_CUDA(attr.get(current_device(), [] {
+            const cudaError_t e = cudaFuncSetAttribute(coarse_tail_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            return e != cudaSuccess ? e : cudaFuncSetAttribute(coarse_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TAIL_BYTES);
+        }));
         if (launch_pdl(coarse_tail_kernel, dim3(TAIL_BLOCKS), dim3(TAIL_THREADS), sizeof(float) * (size_t)(cells + 2 * held), st, ta, S)) return 1;
         CB_CHECK_LAUNCH();
     }
