@@ -681,10 +681,11 @@ __global__ void __launch_bounds__(1024) cgs_kernel(Op A, KArgs a) {
             alpha = beta = 0.;   // restart from the true residual, in the range of a singular A
             first = true;
             best = t[0];
-            if (a.project) {
-                for (long long c = t0; c < N; c += T) v.r[c] = v.r[c] - sg * S[c] * (t[2] / (double)N);
-                grid.sync();     // the update deals the cells out in groups of W: r's next reader is another thread
-            }
+            if (a.project)   // by the thread whose update reads the cell next
+                cg_groups<W>(v.n, false, [&](int c) {
+#pragma unroll
+                    for (int m = 0; m < W; ++m) v.r[c + m] = v.r[c + m] - sg * S[c + m] * (t[2] / (double)N);
+                });
         } else
             first = false;
     }
