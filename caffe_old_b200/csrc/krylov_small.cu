@@ -356,6 +356,7 @@ __global__ void __launch_bounds__(SB) small_cg_kernel(Op op, SmallArgs a) {
 #pragma unroll
     for (int k = 0; k < C; ++k) r[k] = p[k] = q[k] = 0.;
     f.each([&](int k, int l) { r[k] = f.b[l]; });
+    const double growth = a.project ? CG_GROWTH : 1e300;   // NaN counts as growth
     double alpha = 0., beta = 0., best = f.bb;
     bool first = true;
     while (!f.done) {
@@ -380,7 +381,7 @@ __global__ void __launch_bounds__(SB) small_cg_kernel(Op op, SmallArgs a) {
         beta = next * d[0] > 0. ? next / d[0] : 0.;
         const bool broke = d[0] == 0. || d[2] == 0. || alpha != alpha || beta != beta, stuck = broke && first;
         if (d[1] < best) best = d[1];
-        if ((!first && (d[1] <= f.tol2 || f.it >= a.maxit)) || d[1] != d[1] || (a.project && d[1] > CG_GROWTH * best) || broke) {
+        if ((!first && (d[1] <= f.tol2 || f.it >= a.maxit)) || !(d[1] <= growth * best) || broke) {
             double rr;
             f.check(r, a.maxit, rr);
             if (!f.done && stuck) { f.done = true; f.status = 2; }   // no direction from a fresh residual
