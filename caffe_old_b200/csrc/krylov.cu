@@ -712,6 +712,11 @@ __global__ void __launch_bounds__(1024) cgs_kernel(Op A, KArgs a) {
 // 4719 and 5690 iterations a step, 66 and 76 ms): FP32 to 1e-6 and restarted, stalled in every
 // solve, then the FP64 solve, 0.5-1.2 s; FP32 with reliable updates 24829 and 23281 iterations, 547
 // and 266 ms; FP64 vectors on the FP32 matrix 12772 and 10529, 171 and 160 ms.
+//
+// Both figures measured on a skewed 128^3 cavity (3 steps, 5724 iterations) and on one of 64x60x56 cells in a
+// box of 1 x 0.02 x 0.2 (4 steps, 91,740), ms of the p' solves.  MX_DROP 0.5: 100 and 484; 0.2: 96 and 506; 0.05: 94 and
+// 591; 0.01: 94 and 736; 0.001: 101 and 590.  Patience 300 leaves four of the second cavity's eight solves
+// to FP64 (1104 ms); 3000 changes neither (94 and 606) and takes longer to give up.
 constexpr double MX_DROP = 0.05;
 constexpr int MX_PATIENCE = 1000;
 
