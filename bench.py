@@ -19,7 +19,7 @@ as a fallback).  The same steps from rest are also run with the plain FP64 press
 One JSON line on rank 0.  The CPU numbers (--impl reference, and cpu_baseline in the GPU line)
 time the CPU restatement of the reference path (the reference itself needs MPI, PETSc and Boost,
 which this image lacks) on the host cores.  A step of the 25.2M-cell case does not fit a CPU
-budget of minutes (about 57,000 FP64 Krylov iterations per step), so they time whole steps of the
+budget of minutes (about 34,000 FP64 Krylov iterations per step), so they time whole steps of the
 same case on a smaller lattice and say so; nothing is extrapolated.  The GPU line adds the GPU on
 that same smaller lattice, and a fully measured 128^3 cavity (configuration 2) on both.
 """

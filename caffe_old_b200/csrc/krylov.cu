@@ -16,7 +16,8 @@
 // convergence decision and the result is bit-reproducible.  The loop ends on the true
 // residual ||b - A x|| <= rtol ||b|| (checked when the recursive residual meets it; the
 // iteration restarts from the true residual otherwise) or at maxit, so no launch can run
-// unbounded.  Systems of at most 32768 rows run inside one cluster (krylov_small.cu).
+// unbounded.  Lattices of at most 32768 cells, and compressed rows as far as they are short and few, run
+// inside one cluster (krylov_small.cu).
 //
 // Values written earlier in the same launch by other blocks are read with ordinary loads
 // after a reduction or barrier (whose release/acquire pair orders them), never through the

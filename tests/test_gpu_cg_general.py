@@ -49,3 +49,15 @@ def test_the_scaled_form_takes_the_rest(shape, sign):
     assert rc == 0 and rr <= 1e-12
     assert seven_point_residual(shape, coef, x, b) <= 1e-11
     assert not np.array_equal(x, xg) and np.linalg.norm(x - xg) <= 1e-9 * np.linalg.norm(xg)
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_bicgstab_without_allocation_on_the_grid(shape):
+    """The same kernel on the other entry's workspace: same bits."""
+    coef, b = seven_point_system(shape, 6, False)
+    L = _lib.lib()
+    rc, x, its, rr = solve_with(L.caffe_ksp7_solve_device, shape, coef, b, "bicgstab_jacobi")
+    rg, xg, itg, _ = solve_with(L.caffe_ksp7_solve_device_noalloc, shape, coef, b, "bicgstab_jacobi")
+    assert rc == 0 and rg == 0 and rr <= 1e-12 and its == itg
+    assert seven_point_residual(shape, coef, x, b) <= 1e-11
+    assert np.array_equal(x, xg)
