@@ -23,11 +23,10 @@ namespace cb {
 
 constexpr double BI_FLOOR = 3.4694469519536142e-18;   // 2^-58
 
-// rho = (rp, r), rp2 = (rp, rp), rr = (r, r).  The squares decide nearly always; the root where they come close,
+// rho = (rp, r), rp2 = (rp, rp), rr = (r, r).  The squares decide nearly always; the roots where they come close,
 // underflow or overflow.
 __device__ __forceinline__ bool bi_sound(double rho, double rp2, double rr) {
-    const double m = rp2 * fabs(rr);
-    return rho * rho > 2. * BI_FLOOR * BI_FLOOR * m || fabs(rho) > BI_FLOOR * sqrt(m);
+    return rho * rho > 2. * BI_FLOOR * BI_FLOOR * (rp2 * fabs(rr)) || fabs(rho) > BI_FLOOR * (sqrt(rp2) * sqrt(fabs(rr)));
 }
 
 }  // namespace cb

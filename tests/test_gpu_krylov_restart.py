@@ -125,3 +125,17 @@ def test_bicgstab_of_a_singular_system_ignores_the_mean_of_its_right_hand_side(n
     assert st0["p_res_max"] <= 1e-8 and st1["p_res_max"] <= 1e-8
     assert st1["p_iters_last"] <= 1.2 * st0["p_iters_last"] + 5
     assert np.linalg.norm(x1 - x0) <= 1e-4 * np.linalg.norm(x0)
+
+
+@pytest.mark.parametrize("method", ["bicgstab_jacobi"])
+@pytest.mark.parametrize("shape", [(20, 20, 20), (36, 32, 32)])
+def test_right_hand_sides_of_any_size_take_the_same_iterations(shape, method):
+    """Scaled by a power of two every number of a solve scales exactly, up to where the square of a squared norm
+    leaves the range: the restart rules must not see the difference."""
+    coef, b = seven_point_system(shape, 8, method == "cg_jacobi")
+    x, its, _, st = _lib.ksp7_solve(shape, coef, b, method, 1e-10, 5000)
+    assert st == 0
+    for e in (-300, 300):
+        xs, itss, _, st = _lib.ksp7_solve(shape, coef, b * 2.0**e, method, 1e-10, 5000)
+        assert st == 0 and itss == its
+        assert np.array_equal(xs, x * 2.0**e)
