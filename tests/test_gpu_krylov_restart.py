@@ -127,7 +127,7 @@ def test_bicgstab_of_a_singular_system_ignores_the_mean_of_its_right_hand_side(n
     assert np.linalg.norm(x1 - x0) <= 1e-4 * np.linalg.norm(x0)
 
 
-@pytest.mark.parametrize("method", ["bicgstab_jacobi"])
+@pytest.mark.parametrize("method", ["bicgstab_jacobi", "cg_jacobi"])
 @pytest.mark.parametrize("shape", [(20, 20, 20), (36, 32, 32)])
 def test_right_hand_sides_of_any_size_take_the_same_iterations(shape, method):
     """Scaled by a power of two every number of a solve scales exactly, up to where the square of a squared norm
