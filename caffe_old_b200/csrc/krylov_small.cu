@@ -377,8 +377,7 @@ __global__ void __launch_bounds__(SB) small_cg_kernel(Op op, SmallArgs a) {
         f.sum(f.cl, s4, d);
         if (!first) f.it += 1;
         alpha = d[0] / d[2];
-        const double next = (alpha * alpha * d[3] - d[0]) / d[0];   // of one sign with d[0] when sound
-        beta = next > 0. ? next : 0.;
+        beta = (alpha * alpha * d[3] - d[0]) / d[0];   // negative where (r, z) changes sign: 1/d need not be of one sign here
         const bool broke = d[0] == 0. || d[2] == 0. || alpha != alpha || beta != beta, stuck = broke && first;
         if (d[1] < best) best = d[1];
         if ((!first && (d[1] <= f.tol2 || f.it >= a.maxit)) || !(d[1] <= growth * best) || broke) {

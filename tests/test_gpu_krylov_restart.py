@@ -139,3 +139,23 @@ def test_right_hand_sides_of_any_size_take_the_same_iterations(shape, method):
         xs, itss, _, st = _lib.ksp7_solve(shape, coef, b * 2.0**e, method, 1e-10, 5000)
         assert st == 0 and itss == its
         assert np.array_equal(xs, x * 2.0**e)
+
+
+@pytest.mark.parametrize("shape", [(5, 4, 3), (10, 10, 10), (20, 20, 20), (32, 32, 32), (36, 32, 32)])
+@pytest.mark.parametrize("kind", ["zero entry", "one sign turned", "a strip turned", "random signs"])
+def test_cg_with_a_diagonal_that_is_not_of_one_sign(shape, kind):
+    """(r, D^-1 r) changes sign there and beta with it.  Up to 180 iterations; ten times that are allowed."""
+    coef, b = seven_point_system(shape, 8, True)
+    N = b.size
+    if kind == "zero entry":
+        coef[0, 7] = 0.0
+    elif kind == "one sign turned":
+        coef[0, N // 2] *= -1.0
+    elif kind == "a strip turned":
+        coef[0, :N // 8] *= -1.0
+    else:
+        coef[1:] *= 0.3
+        coef[0] *= np.where(np.random.default_rng(8).random(N) < 0.3, -1.0, 1.0)
+    x, _, rr, st = _lib.ksp7_solve(shape, coef, b, "cg_jacobi", 1e-10, 1800)
+    assert st == 0 and rr <= 1e-10
+    assert seven_point_residual(shape, coef, x, b) <= 1.1e-10
